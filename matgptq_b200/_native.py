@@ -89,6 +89,19 @@ def load() -> ctypes.CDLL:
     return lib
 
 
+def load_torch_ops():
+    """The C++ module that registers ``torch.ops.matgptq_cuda.*``, bound to the library above. Raises if it is missing."""
+    load()
+    try:
+        from . import _torch_ops
+    except ImportError as e:
+        raise ImportError(
+            f"the operator module of matgptq_b200 is not built ({e}). Run `python -m matgptq_b200.build`; there is no "
+            "fallback.") from e
+    _torch_ops.bind(_LIB_PATH)
+    return _torch_ops
+
+
 def device_status(reset: bool = True) -> int:
     """First failure code recorded by a kernel on the current device (0 = none); synchronises."""
     out = ctypes.c_int(0)

