@@ -56,10 +56,10 @@ int slice_launch(const uint8_t *in, uint8_t *out, long long numel, int master_bi
 }
 
 // ---------------------------------------------------------------------------
-// packing: one thread builds the 2*b words that one lane will later decode
+// packing: one thread builds the 2*b words that one lane will later decode (pack_lane on the host)
 // ---------------------------------------------------------------------------
 template <int B>
-MG_HD void pack_lane(const uint8_t *codes, int K, int tile, int kb, int lane, int slice_from_master,
+static void pack_lane(const uint8_t *codes, int K, int tile, int kb, int lane, int slice_from_master,
                      uint32_t (&w)[2 * B]) {
   for (int j = 0; j < 2 * B; ++j) w[j] = 0u;
   const int g = lane >> 2, t = lane & 3;
@@ -78,20 +78,89 @@ MG_HD void pack_lane(const uint8_t *codes, int K, int tile, int kb, int lane, in
   }
 }
 
+// Four codes at once: mask to B bits, or slice from the master (matryoshka_slice() on every byte of the word).  The
+// rounded value is at most 2^B, which fits the byte for B < 8, so no carry crosses a byte.
+template <int B> __device__ __forceinline__ uint32_t slice4(uint32_t x, int slice_from_master) {
+  constexpr uint32_t kOnes = 0x01010101u, kMask = ((1u << B) - 1u) * kOnes;
+  if (slice_from_master == 0) return x & kMask;
+  if constexpr (B == 8) {
+    return x;
+  } else {
+    uint32_t v = (x >> (8 - B)) & kMask;
+    if (slice_from_master != B) {
+      v += (x >> (7 - B)) & kOnes;  // the rounding bit
+      v -= (v >> B) & kOnes;        // saturate: 2^B becomes 2^B - 1
+    }
+    return v;
+  }
+}
+
+// One warp packs one block of 16 x 128 codes, as it will later be decoded: a lane reads 8 consecutive codes of rows g
+// and g+8 in each of four 32-wide chunks (8-byte loads that fill whole 32-byte sectors), slices four bytes per
+// instruction, spreads two codes over the halves of a word with one PRMT, and writes its words as 16-byte vectors.
+// Bound by HBM (one byte in, B/8 out per code).  The byte-wise form it replaces needed 64 one-byte loads and 64
+// scalar slices a lane: 14336 x 4096 from 8 to 3 bits: 61.4 -> 18.4 us on B200 (80.7 MB, 4.4 TB/s; a copy of as many
+// bytes at the measured peak takes 12.5 us).
 template <int B>
-__global__ void pack_kernel(const uint8_t *__restrict__ codes, uint32_t *__restrict__ packed, int tiles, int kblocks,
-                            int K, int slice_from_master) {
+__global__ void __launch_bounds__(256) pack_kernel(const uint8_t *__restrict__ codes, uint32_t *__restrict__ packed, int tiles,
+                                                   int kblocks, int K, int slice_from_master) {
   const long long gid = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   const long long nblocks = static_cast<long long>(tiles) * kblocks;
   const long long blk = gid >> 5;
   const int lane = static_cast<int>(gid & 31);
   if (blk >= nblocks) return;
-  const int tile = static_cast<int>(blk / kblocks), kb = static_cast<int>(blk % kblocks);
-  uint32_t w[2 * B];
-  pack_lane<B>(codes, K, tile, kb, lane, slice_from_master, w);
-  uint32_t *dst = packed + blk * BlockTraits<B>::WORDS;
+  const int tile = static_cast<int>(blk / kblocks), kb = static_cast<int>(blk - static_cast<long long>(tile) * kblocks);
+  const int g = lane >> 2, t = lane & 3;
+  const uint8_t *src = codes + (static_cast<size_t>(tile) * 16 + g) * K + kb * 128 + 8 * t;
+  uint32_t c[2][8];  // [row g, g+8][k-step]: four consecutive codes
+  if ((reinterpret_cast<uintptr_t>(codes) & 7u) == 0) {
 #pragma unroll
-  for (int j = 0; j < 2 * B; ++j) dst[word_slot<B>(lane, j)] = w[j];
+    for (int jj = 0; jj < 4; ++jj)
+#pragma unroll
+      for (int rr = 0; rr < 2; ++rr) {
+        const uint2 q = *reinterpret_cast<const uint2 *>(src + static_cast<size_t>(8 * rr) * K + 32 * jj);
+        c[rr][2 * jj] = q.x;
+        c[rr][2 * jj + 1] = q.y;
+      }
+  } else {  // a caller's buffer may start anywhere
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+      for (int rr = 0; rr < 2; ++rr) {
+        const uint8_t *p = src + static_cast<size_t>(8 * rr) * K + 32 * (i >> 1) + 4 * (i & 1);
+        c[rr][i] = p[0] | (static_cast<uint32_t>(p[1]) << 8) | (static_cast<uint32_t>(p[2]) << 16) | (static_cast<uint32_t>(p[3]) << 24);
+      }
+  }
+  uint32_t w[2 * B];
+#pragma unroll
+  for (int j = 0; j < 2 * B; ++j) w[j] = 0u;
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int rr = 0; rr < 2; ++rr) {
+      const uint32_t v = slice4<B>(c[rr][i], slice_from_master);
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const uint32_t pair = __byte_perm(v, 0u, e ? 0x4342 : 0x4140);  // codes 2e and 2e+1 in the low and high half
+        Piece pc[3];
+        const int n = code_pieces<B>(4 * i + 2 * e + rr, 0, pc);
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+          if (k < n) w[pc[k].word] |= ((pair >> pc[k].cshift) & (((1u << pc[k].nbits) - 1u) * 0x00010001u)) << pc[k].off;
+      }
+    }
+  uint32_t *dst = packed + blk * BlockTraits<B>::WORDS;
+  if ((reinterpret_cast<uintptr_t>(packed) & 15u) != 0) {
+#pragma unroll
+    for (int j = 0; j < 2 * B; ++j) dst[word_slot<B>(lane, j)] = w[j];
+    return;
+  }
+#pragma unroll
+  for (int v = 0; v < BlockTraits<B>::NV; ++v)
+    *reinterpret_cast<uint4 *>(dst + v * 128 + lane * 4) = make_uint4(w[4 * v], w[4 * v + 1], w[4 * v + 2], w[4 * v + 3]);
+  if constexpr (BlockTraits<B>::TAIL == 2)
+    *reinterpret_cast<uint2 *>(dst + BlockTraits<B>::NV * 128 + lane * 2) =
+        make_uint2(w[4 * BlockTraits<B>::NV], w[4 * BlockTraits<B>::NV + 1]);
 }
 
 template <int B>
@@ -100,7 +169,7 @@ static int pack_launch_b(const uint8_t *codes, uint32_t *packed, int N, int K, i
   const int tiles = N / 16, kblocks = K / 128;
   const long long threads_total = static_cast<long long>(tiles) * kblocks * 32;
   if (threads_total == 0) return MG_OK;
-  const int threads = 128;
+  const int threads = 256;
   const long long blocks = (threads_total + threads - 1) / threads;
   pack_kernel<B><<<static_cast<unsigned>(blocks), threads, 0, stream>>>(codes, packed, tiles, kblocks, K, slice_from_master);
   return cudaGetLastError() == cudaSuccess ? MG_OK : MG_ERR_CUDA;
