@@ -10,42 +10,12 @@
 #include <cstdint>
 
 #include "../../include/matgptq_b200.h"
+#include "helper_kernels.cuh"
 #include "kernels.h"
 
 namespace mg {
 
-template <typename T> __device__ __forceinline__ float to_f(T v);
-template <> __device__ __forceinline__ float to_f<__half>(__half v) { return __half2float(v); }
-template <> __device__ __forceinline__ float to_f<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
-template <typename T> __device__ __forceinline__ T from_f(float v);
-template <> __device__ __forceinline__ __half from_f<__half>(float v) { return __float2half_rn(v); }
-template <> __device__ __forceinline__ __nv_bfloat16 from_f<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
-
 // x[row] += delta[row] (when delta != null), then h[row] = rmsnorm(x[row]) * weight.  One CTA per row.
-// Programmatic dependent launch: let the next kernel of the stream start its prologue now (the packed products
-// prefetch their weights there), then wait until the previous kernel's results are complete and visible.  Both
-// are no-ops for a kernel that was launched without the attribute and has no dependents.
-__device__ __forceinline__ void pdl_prologue() {
-  asm volatile("griddepcontrol.launch_dependents;");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-
-template <typename Kernel, typename... Args>
-static int launch_helper(Kernel kernel, unsigned grid, unsigned block, cudaStream_t stream, bool pdl, Args... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid, 1, 1);
-  cfg.blockDim = dim3(block, 1, 1);
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  if (pdl) {
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-  }
-  return cudaLaunchKernelEx(&cfg, kernel, args...) == cudaSuccess ? MG_OK : MG_ERR_CUDA;
-}
-
 template <typename T>
 __global__ void __launch_bounds__(256) add_rmsnorm_kernel(T *__restrict__ x, const T *__restrict__ delta, const T *__restrict__ weight,
                                                           T *__restrict__ h, int hidden, float eps) {
@@ -168,6 +138,43 @@ __global__ void rope_kv_kernel(const T *__restrict__ qkv, const long long *__res
   }
 }
 
+// The same with 16-byte accesses: a thread takes eight elements (four pairs) of one head, blockIdx.y walks the rows.
+// head_dim % 8 == 0, everything 16-byte aligned.  Bound by latency for few rows and by memory for a prompt; one pair per
+// thread spent its time on three 64-bit divisions and 2-byte accesses (with silu_mul below, four 8B layers: a prompt of 512
+// tokens 1462 -> 1388 us, a decode step at batch 1 258 -> 253).
+template <typename T>
+__global__ void __launch_bounds__(256) rope_kv_vec_kernel(const T *__restrict__ qkv, const long long *__restrict__ positions,
+                                                          const float *__restrict__ cos_t, const float *__restrict__ sin_t,
+                                                          T *__restrict__ q_out, T *__restrict__ k_cache, T *__restrict__ v_cache,
+                                                          int B, int S, int H, int KV, int d, int max_seq) {
+  pdl_prologue();
+  const int heads = H + 2 * KV, vecs = d >> 3;
+  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+  if (idx >= heads * vecs) return;
+  const int head = idx / vecs, i = (idx - head * vecs) * 8;
+  for (int row = blockIdx.y; row < B * S; row += gridDim.y) {
+    const int b = row / S, s = row - b * S;
+    const long long pos = positions[s];
+    uint4 v = *reinterpret_cast<const uint4 *>(qkv + (static_cast<size_t>(row) * heads + head) * d + i);
+    if (head < H + KV) {
+      const float4 cs = *reinterpret_cast<const float4 *>(cos_t + pos * (d >> 1) + (i >> 1));
+      const float4 sn = *reinterpret_cast<const float4 *>(sin_t + pos * (d >> 1) + (i >> 1));
+      const float cv[4] = {cs.x, cs.y, cs.z, cs.w}, sv[4] = {sn.x, sn.y, sn.z, sn.w};
+      T *e = reinterpret_cast<T *>(&v);
+#pragma unroll
+      for (int p = 0; p < 4; ++p) {
+        const float a = to_f(e[2 * p]), c = to_f(e[2 * p + 1]);
+        e[2 * p] = from_f<T>(a * cv[p] - c * sv[p]);
+        e[2 * p + 1] = from_f<T>(a * sv[p] + c * cv[p]);
+      }
+    }
+    T *dst = head < H ? q_out + ((static_cast<size_t>(b) * H + head) * S + s) * d
+             : head < H + KV ? k_cache + ((static_cast<size_t>(b) * KV + (head - H)) * max_seq + pos) * d
+                             : v_cache + ((static_cast<size_t>(b) * KV + (head - H - KV)) * max_seq + pos) * d;
+    *reinterpret_cast<uint4 *>(dst + i) = v;
+  }
+}
+
 // gu [rows, 2*inter] -> out [rows, inter] = silu(gate) * up, both factors rounded to the model dtype first
 template <typename T>
 __global__ void silu_mul_kernel(const T *__restrict__ gu, T *__restrict__ out, long long rows, int inter) {
@@ -180,6 +187,29 @@ __global__ void silu_mul_kernel(const T *__restrict__ gu, T *__restrict__ out, l
     const float gte = to_f(gu[r * 2 * inter + c]), up = to_f(gu[r * 2 * inter + inter + c]);
     const float act = to_f(from_f<T>(gte / (1.f + __expf(-gte))));
     out[idx] = from_f<T>(act * up);
+  }
+}
+
+// The same with 16-byte accesses, eight outputs a thread, blockIdx.y walks the rows: inter % 8 == 0 and 16-byte aligned
+// buffers.  Bound by memory for a prompt; one output per thread spent its time on a 64-bit division and 2-byte accesses.
+template <typename T>
+__global__ void __launch_bounds__(256) silu_mul_vec_kernel(const T *__restrict__ gu, T *__restrict__ out, long long rows, int inter) {
+  pdl_prologue();
+  const int c = (blockIdx.x * blockDim.x + threadIdx.x) * 8;
+  if (c >= inter) return;
+  for (long long r = blockIdx.y; r < rows; r += gridDim.y) {
+    const uint4 gv = *reinterpret_cast<const uint4 *>(gu + r * 2 * inter + c);
+    const uint4 uv = *reinterpret_cast<const uint4 *>(gu + r * 2 * inter + inter + c);
+    const T *ge = reinterpret_cast<const T *>(&gv);
+    const T *ue = reinterpret_cast<const T *>(&uv);
+    uint4 o;
+    T *oe = reinterpret_cast<T *>(&o);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const float gte = to_f(ge[k]);
+      oe[k] = from_f<T>(to_f(from_f<T>(gte / (1.f + __expf(-gte)))) * to_f(ue[k]));
+    }
+    *reinterpret_cast<uint4 *>(out + r * inter + c) = o;
   }
 }
 
@@ -244,6 +274,15 @@ static unsigned grid_for(long long total, int threads) {
   return static_cast<unsigned>(blocks);
 }
 
+// blockIdx.x over the vectors of a row, blockIdx.y over the rows (a few rows a block once the grid fills the GPU)
+static dim3 rows_grid(long long vecs, long long rows) {
+  const unsigned x = static_cast<unsigned>((vecs + 255) / 256);
+  long long y = (148LL * 64 + x - 1) / x;
+  if (y > rows) y = rows;
+  if (y > 65535) y = 65535;
+  return dim3(x, static_cast<unsigned>(y), 1);
+}
+
 }  // namespace mg
 
 extern "C" {
@@ -256,7 +295,7 @@ int matgptq_b200_add_rmsnorm(void *x, const void *delta, const void *weight, voi
   const bool vec = hidden % 8 == 0 && hidden <= static_cast<int64_t>(mg::kNormThreads) * 8 * mg::kRowVecs &&
                    (reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(delta) | reinterpret_cast<uintptr_t>(weight) |
                     reinterpret_cast<uintptr_t>(h)) % 16 == 0;
-  const unsigned grid = static_cast<unsigned>(rows);
+  const dim3 grid(static_cast<unsigned>(rows));
   const int hd = static_cast<int>(hidden);
   const bool pdl = (flags & MATGPTQ_B200_FLAG_PDL) != 0;
   if (flags & MATGPTQ_B200_FLAG_BF16) {
@@ -286,19 +325,24 @@ int matgptq_b200_rope_kv(const void *qkv, const int64_t *positions, const float 
   const long long total = batch * seq * (n_heads + 2 * n_kv_heads) * (head_dim / 2);
   if (total <= 0) return MG_OK;
   cudaStream_t cs = static_cast<cudaStream_t>(stream);
-  const unsigned grid = mg::grid_for(total, 256);
   const long long *pos = reinterpret_cast<const long long *>(positions);
-  if (flags & MATGPTQ_B200_FLAG_BF16)
-    return mg::launch_helper(mg::rope_kv_kernel<__nv_bfloat16>, grid, 256, cs, (flags & MATGPTQ_B200_FLAG_PDL) != 0,
-        static_cast<const __nv_bfloat16 *>(qkv), pos, cos_table, sin_table, static_cast<__nv_bfloat16 *>(q_out),
-        static_cast<__nv_bfloat16 *>(k_cache), static_cast<__nv_bfloat16 *>(v_cache), static_cast<int>(batch), static_cast<int>(seq),
-        static_cast<int>(n_heads), static_cast<int>(n_kv_heads), static_cast<int>(head_dim), static_cast<int>(max_seq));
-  else
-    return mg::launch_helper(mg::rope_kv_kernel<__half>, grid, 256, cs, (flags & MATGPTQ_B200_FLAG_PDL) != 0,
-        static_cast<const __half *>(qkv), pos, cos_table, sin_table, static_cast<__half *>(q_out), static_cast<__half *>(k_cache),
-        static_cast<__half *>(v_cache), static_cast<int>(batch), static_cast<int>(seq), static_cast<int>(n_heads),
-        static_cast<int>(n_kv_heads), static_cast<int>(head_dim), static_cast<int>(max_seq));
-  return cudaGetLastError() == cudaSuccess ? MG_OK : MG_ERR_CUDA;
+  const bool vec = head_dim % 8 == 0 && batch * seq <= INT32_MAX && n_heads + 2 * n_kv_heads <= (1 << 16) && head_dim <= (1 << 12) &&
+                   (reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(cos_table) | reinterpret_cast<uintptr_t>(sin_table) |
+                    reinterpret_cast<uintptr_t>(q_out) | reinterpret_cast<uintptr_t>(k_cache) | reinterpret_cast<uintptr_t>(v_cache)) % 16 == 0;
+  const dim3 grid = vec ? mg::rows_grid((n_heads + 2 * n_kv_heads) * (head_dim / 8), batch * seq) : dim3(mg::grid_for(total, 256));
+  auto go = [&](auto kernel, auto tag) {
+    using T = decltype(tag);
+    return mg::launch_helper(kernel, grid, 256, cs, (flags & MATGPTQ_B200_FLAG_PDL) != 0, static_cast<const T *>(qkv), pos, cos_table,
+                             sin_table, static_cast<T *>(q_out), static_cast<T *>(k_cache), static_cast<T *>(v_cache),
+                             static_cast<int>(batch), static_cast<int>(seq), static_cast<int>(n_heads), static_cast<int>(n_kv_heads),
+                             static_cast<int>(head_dim), static_cast<int>(max_seq));
+  };
+  if (flags & MATGPTQ_B200_FLAG_BF16) {
+    using T = __nv_bfloat16;
+    return vec ? go(mg::rope_kv_vec_kernel<T>, T{}) : go(mg::rope_kv_kernel<T>, T{});
+  }
+  using T = __half;
+  return vec ? go(mg::rope_kv_vec_kernel<T>, T{}) : go(mg::rope_kv_kernel<T>, T{});
 }
 
 int matgptq_b200_argmax(const void *logits, int64_t *out, int64_t rows, int64_t cols, uint32_t flags, void *stream) {
@@ -320,16 +364,20 @@ int matgptq_b200_silu_mul(const void *gate_up, void *out, int64_t rows, int64_t 
   if (!gate_up || !out || rows < 0 || intermediate <= 0) return MG_ERR_BAD_ARG;
   if (rows == 0) return MG_OK;
   cudaStream_t cs = static_cast<cudaStream_t>(stream);
-  const unsigned grid = mg::grid_for(rows * intermediate, 256);
-  if (flags & MATGPTQ_B200_FLAG_BF16)
-    return mg::launch_helper(mg::silu_mul_kernel<__nv_bfloat16>, grid, 256, cs, (flags & MATGPTQ_B200_FLAG_PDL) != 0,
-                             static_cast<const __nv_bfloat16 *>(gate_up), static_cast<__nv_bfloat16 *>(out),
-                             static_cast<long long>(rows), static_cast<int>(intermediate));
-  else
-    return mg::launch_helper(mg::silu_mul_kernel<__half>, grid, 256, cs, (flags & MATGPTQ_B200_FLAG_PDL) != 0,
-                             static_cast<const __half *>(gate_up), static_cast<__half *>(out), static_cast<long long>(rows),
-                             static_cast<int>(intermediate));
-  return cudaGetLastError() == cudaSuccess ? MG_OK : MG_ERR_CUDA;
+  const bool vec = intermediate % 8 == 0 && intermediate <= (1 << 24) &&
+                   (reinterpret_cast<uintptr_t>(gate_up) | reinterpret_cast<uintptr_t>(out)) % 16 == 0;
+  const dim3 grid = vec ? mg::rows_grid(intermediate / 8, rows) : dim3(mg::grid_for(rows * intermediate, 256));
+  auto go = [&](auto kernel, auto tag) {
+    using T = decltype(tag);
+    return mg::launch_helper(kernel, grid, 256, cs, (flags & MATGPTQ_B200_FLAG_PDL) != 0, static_cast<const T *>(gate_up),
+                             static_cast<T *>(out), static_cast<long long>(rows), static_cast<int>(intermediate));
+  };
+  if (flags & MATGPTQ_B200_FLAG_BF16) {
+    using T = __nv_bfloat16;
+    return vec ? go(mg::silu_mul_vec_kernel<T>, T{}) : go(mg::silu_mul_kernel<T>, T{});
+  }
+  using T = __half;
+  return vec ? go(mg::silu_mul_vec_kernel<T>, T{}) : go(mg::silu_mul_kernel<T>, T{});
 }
 
 }  // extern "C"
