@@ -58,7 +58,7 @@ struct GemmParams {
   int kblocks;  // K / 128
   float *partial;  // null: the CTAs along K add their sums inside a cluster; else [split][M][N] fp32 scratch for them
   int split;    // CTAs along K
-  int ncols;    // UMMA N: batch rows per pass rounded up to 16
+  int ncols;    // UMMA N: batch rows of a CTA, a multiple of 16
   int stages;
 };
 
@@ -294,8 +294,8 @@ __device__ __forceinline__ void gemm_tc_body(const GemmParams &p, const CUtensor
   volatile uint32_t *tmem_slot = reinterpret_cast<volatile uint32_t *>(base + 17 * 8);
 
   const int sk = blockIdx.y;
-  const int m0 = blockIdx.z * 256;
-  const int mrows = min(p.M - m0, 256);
+  const int m0 = blockIdx.z * p.ncols;
+  const int mrows = min(p.M - m0, p.ncols);
   const int kb_lo = sk * p.kblocks / p.split;
   const int kb_hi = (sk + 1) * p.kblocks / p.split;
   const int nblk = kb_hi - kb_lo;
@@ -714,7 +714,10 @@ static int launch_gemm_tc_warps(GemmParams p, cudaStream_t stream, bool pdl, flo
 // are no more CTAs than SMs.
 template <int B, int GS, bool BF16>
 static int launch_gemm_tc(GemmParams p, cudaStream_t stream, bool pdl, float *fallback_partial) {
-  p.ncols = round_up16(p.M < 256 ? p.M : 256);
+  // The batch goes in as few blocks of at most 256 rows as it takes, all of one size: a last block that is mostly empty
+  // costs as much as a full one (300 rows as 2 x 160 instead of 256 + 44 in 256 columns: 8192 x 8192, 8 bits 71.0 -> 63.0 us).
+  const int blocks = (p.M + 255) / 256;
+  p.ncols = round_up16((p.M + blocks - 1) / blocks);
   int sm_count = 0;
   {
     const int st = current_device_sm_count(&sm_count);

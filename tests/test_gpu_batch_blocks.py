@@ -1,0 +1,32 @@
+"""Batches of several blocks on the tensor-core path, at the edges of the blocks: integer-valued weights and activations make
+every sum exact, so the product of the dense weights in fp64 is the expected result bit for bit."""
+import pytest
+import torch
+
+from matgptq_b200 import _native, ops  # noqa: F401
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("b,gs,n_out,n_in,m", [
+    (4, 128, 128, 256, 257),     # two blocks of 144, the last 15 short
+    (2, 32, 272, 512, 288),      # two full blocks of 144
+    (8, -1, 2064, 640, 300),     # 2 x 160
+    (3, 128, 1024, 4096, 512),   # full blocks, K split
+    (6, 128, 4096, 1024, 513),   # three blocks of 176
+    (4, 128, 14336, 256, 1025)])
+def test_blocks_of_a_batch(cuda, dtype, b, gs, n_out, n_in, m):
+    gen = torch.Generator(device=cuda).manual_seed(m)
+    flag = 1 | (2 if dtype == torch.bfloat16 else 0)
+    q = torch.randint(0, 256, (n_out, n_in), generator=gen, device=cuda, dtype=torch.uint8)
+    # scales are powers of two: weights are multiples of 2^-7 of size up to 2, sums stay below 2^24 such steps
+    scales = torch.full((n_out, 1 if gs == -1 else n_in // gs), 2.0 ** -6, device=cuda, dtype=dtype)
+    scales[::3] *= 0.5
+    x = torch.randint(-2, 3, (m, n_in), generator=gen, device=cuda).to(dtype)
+    packed = torch.ops.matgptq_cuda.slice_pack_matgptq_qweights(q, n_out, n_in, 8, b, gs, flag)
+    s = torch.ops.matgptq_cuda.reorder_matgptq_scales(scales, n_out, n_in, gs)
+    w = torch.ops.matgptq_cuda.dequantize_matgptq(packed, s, n_out, n_in, b, gs, flag)
+    y = torch.ops.matgptq_cuda.matmul_matgptq(x, packed, s, n_out, n_in, b, gs, flag)
+    assert _native.device_status() == 0
+    assert torch.equal(y, (x.double() @ w.double().t()).to(dtype))
