@@ -104,6 +104,11 @@ __global__ void __launch_bounds__(kNormThreads) add_rmsnorm_vec_kernel(T *__rest
   }
 }
 
+// The rotation with its roundings spelled out: left to the compiler, the two kernels below contracted the same expression
+// differently, and a model whose layers amplify one flipped bit showed it.
+__device__ __forceinline__ float rotated_even(float a, float c, float cs, float sn) { return __fmaf_rn(a, cs, -__fmul_rn(c, sn)); }
+__device__ __forceinline__ float rotated_odd(float a, float c, float cs, float sn) { return __fmaf_rn(c, cs, __fmul_rn(a, sn)); }
+
 // qkv [B, S, (H + 2*KV) * d] -> q_out [B, H, S, d] rotated; k rotated and v written into the caches
 // [B, KV, max_seq, d] at positions[s].  cos/sin are [max_seq, d/2] fp32.  Pairs are (2i, 2i+1).
 template <typename T>
@@ -125,7 +130,7 @@ __global__ void rope_kv_kernel(const T *__restrict__ qkv, const long long *__res
     const float a = to_f(src[0]), c = to_f(src[1]);
     if (head < H + KV) {
       const float cs = cos_t[pos * half + i], sn = sin_t[pos * half + i];
-      const T r0 = from_f<T>(a * cs - c * sn), r1 = from_f<T>(a * sn + c * cs);
+      const T r0 = from_f<T>(rotated_even(a, c, cs, sn)), r1 = from_f<T>(rotated_odd(a, c, cs, sn));
       T *dst = (head < H) ? q_out + ((static_cast<size_t>(b) * H + head) * S + s) * d + 2 * i
                           : k_cache + ((static_cast<size_t>(b) * KV + (head - H)) * max_seq + pos) * d + 2 * i;
       dst[0] = r0;
@@ -164,8 +169,8 @@ __global__ void __launch_bounds__(256) rope_kv_vec_kernel(const T *__restrict__ 
 #pragma unroll
       for (int p = 0; p < 4; ++p) {
         const float a = to_f(e[2 * p]), c = to_f(e[2 * p + 1]);
-        e[2 * p] = from_f<T>(a * cv[p] - c * sv[p]);
-        e[2 * p + 1] = from_f<T>(a * sv[p] + c * cv[p]);
+        e[2 * p] = from_f<T>(rotated_even(a, c, cv[p], sv[p]));
+        e[2 * p + 1] = from_f<T>(rotated_odd(a, c, cv[p], sv[p]));
       }
     }
     T *dst = head < H ? q_out + ((static_cast<size_t>(b) * H + head) * S + s) * d

@@ -59,3 +59,26 @@ def test_rope_kv(lib, cuda, dtype, batch, seq, heads, kv, d, shift):
     assert torch.equal(v[:, :, pos], qkv.transpose(1, 2)[:, heads + kv:])
     others = [i for i in range(max_seq) if i not in pos.tolist()]
     assert not k[:, :, others].any() and not v[:, :, others].any()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_both_access_widths_give_the_same_bits(lib, cuda, dtype):
+    batch, seq, heads, kv, d, max_seq = 2, 512, 32, 8, 128, 512
+    flag, stream = FLAG_BF16 if dtype == torch.bfloat16 else 0, torch.cuda.current_stream().cuda_stream
+    ang = torch.arange(max_seq, device=cuda)[:, None] * 1.7 ** -torch.arange(d // 2, device=cuda)
+    cos, sin, pos = ang.cos().float().contiguous(), ang.sin().float().contiguous(), torch.arange(seq, device=cuda)
+    outs = []
+    for shift in (0, 1):
+        # the same values at both alignments
+        qkv = _shifted((batch, seq, heads + 2 * kv, d), dtype, cuda, 0, 5)
+        if shift:
+            qkv = torch.cat([qkv.new_zeros(1), qkv.flatten()])[1:].view(qkv.shape)
+        q = torch.zeros(batch, heads, seq, d, dtype=dtype, device=cuda)
+        k, v = (torch.zeros(batch, kv, max_seq, d, dtype=dtype, device=cuda) for _ in range(2))
+        assert lib.matgptq_b200_rope_kv(qkv.data_ptr(), pos.data_ptr(), cos.data_ptr(), sin.data_ptr(), q.data_ptr(), k.data_ptr(),
+                                        v.data_ptr(), batch, seq, heads, kv, d, max_seq, flag, stream) == 0
+        act = torch.zeros(batch * seq, (heads + 2 * kv) * d // 2, dtype=dtype, device=cuda)
+        assert lib.matgptq_b200_silu_mul(qkv.data_ptr(), act.data_ptr(), act.shape[0], act.shape[1], flag, stream) == 0
+        outs.append((q, k, v, act))
+    assert all(torch.equal(a, b) for a, b in zip(*outs))
