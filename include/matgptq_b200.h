@@ -63,9 +63,7 @@ int matgptq_b200_matmul(int64_t bitwidth, int64_t group_size, int64_t n_out, int
  * product with per-group zero points, Wdq = s * (code * 2^(8-b) - zero), the formula of dequantize()
  * (src/quant_utils_matgpqt.py:19-22).  `z` holds the zero points in master (8-bit) units, in the type of the
  * scales and in their reordered layout (matgptq_b200_reorder_scales on the [N, G] zero points).  z == NULL is
- * matgptq_b200_matmul.  Batches take the paths of matgptq_b200_matmul: the GEMV family for few rows, the tensor
- * cores above (the dense weights are dequantize()'s, bit for bit; with FLAG_SCRATCH_REDUCE, which needs scratch that this
- * entry does not take, it is ignored).
+ * matgptq_b200_matmul.  Every batch size runs on the GEMV family (more than 16 rows in passes of 16).
  */
 int matgptq_b200_matmul_zp(int64_t bitwidth, int64_t group_size, int64_t n_out, int64_t n_in, int64_t batch,
                            const void *w, const void *s, const void *z, const void *x, void *y, void *stream,

@@ -42,12 +42,11 @@ def _sources() -> list[str]:
 
 
 def _newest_header_mtime() -> float:
-    """Newest header, or source that another source includes (gemv_zp.cu and gemm_tc_zp.cu compile theirs a second
-    time)."""
+    """Newest header, or source that another source includes (gemv_zp.cu compiles gemv.cu a second time)."""
     mt = 0.0
     for d in (CSRC, INCLUDE):
         for name in os.listdir(d):
-            if name.endswith((".h", ".cuh")) or name in ("gemv.cu", "gemm_tc.cu"):
+            if name.endswith((".h", ".cuh")) or name == "gemv.cu":
                 mt = max(mt, os.path.getmtime(os.path.join(d, name)))
     return mt
 

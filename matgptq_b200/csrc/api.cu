@@ -82,21 +82,22 @@ static int matmul_impl(int64_t bitwidth, int64_t group_size, int64_t n_out, int6
   const bool bf16 = (flags & MATGPTQ_B200_FLAG_BF16) != 0;
   const bool pdl = (flags & MATGPTQ_B200_FLAG_PDL) != 0;
   const bool tensor_core = path == 2 || (path == 0 && uses_tensor_cores(n_out, batch));
-  int r = MG_OK;
-  // With zero points the same line holds: the operator is defined over the weights of dequantize(), which the
-  // tensor-core path builds bit for bit (4096 x 4096 at 128 rows, 4 bits, fp16: 52.2 us
-  // in eight passes of the GEMV, 14.2 here).
-  if (tensor_core) {
-    const auto launch = z ? mg::gemm_tc_zp_launch : mg::gemm_tc_launch;
-    r = launch(static_cast<int>(bitwidth), static_cast<int>(group_size), static_cast<int>(n_out), static_cast<int>(n_in),
-               static_cast<int>(batch), w, s, z, x, y, workspace, workspace_bytes, bf16, pdl, split_k, cs, 0,
-               (flags & MATGPTQ_B200_FLAG_SCRATCH_REDUCE) != 0);
-  }
-  if (z && tensor_core && r == MG_ERR_CUDA) (void)cudaGetLastError();  // no cluster on this device and no scratch: the GEMV
-  if (!tensor_core || (z && r == MG_ERR_CUDA)) {
-    const auto launch = z ? mg::gemv_zp_launch : mg::gemv_launch;
-    r = launch(static_cast<int>(bitwidth), static_cast<int>(group_size), static_cast<int>(n_out), static_cast<int>(n_in),
-               static_cast<int>(batch), w, s, z, x, y, bf16, pdl, warps_per_cta, split_k, cs, 0);
+  int r;
+  if (z) {
+    // zero points: every batch size runs on the GEMV family (more than 16 rows in passes of 16), which applies scale and
+    // zero point in fp32; the tensor-core path has the implicit zero point only.  Dense tiles with zero points were 3.7
+    // times as fast at 128 rows, but round s * (code - zero) to 16 bits: 1.4 times the error against 64 bits (K = 4096,
+    // 4 bits: fp16 2.1e-4 -> 3.0e-4, bf16 1.7e-3 -> 2.4e-3), and in fp16 an infinity where that product passes 65504.
+    if (path > 1) return MG_ERR_UNSUPPORTED;
+    r = mg::gemv_zp_launch(static_cast<int>(bitwidth), static_cast<int>(group_size), static_cast<int>(n_out),
+                           static_cast<int>(n_in), static_cast<int>(batch), w, s, z, x, y, bf16, pdl, warps_per_cta, split_k, cs);
+  } else if (tensor_core) {
+    r = mg::gemm_tc_launch(static_cast<int>(bitwidth), static_cast<int>(group_size), static_cast<int>(n_out),
+                           static_cast<int>(n_in), static_cast<int>(batch), w, s, x, y, workspace, workspace_bytes, bf16,
+                           pdl, split_k, cs, 0, (flags & MATGPTQ_B200_FLAG_SCRATCH_REDUCE) != 0);
+  } else {
+    r = mg::gemv_launch(static_cast<int>(bitwidth), static_cast<int>(group_size), static_cast<int>(n_out),
+                        static_cast<int>(n_in), static_cast<int>(batch), w, s, nullptr, x, y, bf16, pdl, warps_per_cta, split_k, cs);
   }
   if (r != MG_OK) return r;
   if (!(flags & MATGPTQ_B200_FLAG_ASYNC)) {
@@ -121,8 +122,7 @@ int matgptq_b200_matmul(int64_t bitwidth, int64_t group_size, int64_t n_out, int
 int matgptq_b200_matmul_zp(int64_t bitwidth, int64_t group_size, int64_t n_out, int64_t n_in, int64_t batch,
                            const void *w, const void *s, const void *z, const void *x, void *y, void *stream,
                            uint32_t flags) {
-  return matmul_impl(bitwidth, group_size, n_out, n_in, batch, w, s, x, y, stream,
-                     z ? flags & ~static_cast<uint32_t>(MATGPTQ_B200_FLAG_SCRATCH_REDUCE) : flags, nullptr, 0, 0, 0, 0, z);
+  return matmul_impl(bitwidth, group_size, n_out, n_in, batch, w, s, x, y, stream, flags, nullptr, 0, 0, 0, 0, z);
 }
 
 int matgptq_b200_matmul_ws(int64_t bitwidth, int64_t group_size, int64_t n_out, int64_t n_in, int64_t batch,
@@ -171,7 +171,7 @@ int matgptq_b200_matmul_grouped(const matgptq_b200_segment *segments, int n_segm
       if (uses_tensor_cores(segments[i].n_out, batch))
         r = mg::gemm_tc_launch(static_cast<int>(segments[i].bitwidth), static_cast<int>(group_size),
                                static_cast<int>(segments[i].n_out), static_cast<int>(n_in), static_cast<int>(batch),
-                               segments[i].w, segments[i].s, nullptr, x, yi, workspace, workspace_bytes, bf16, pdl, 0, cs,
+                               segments[i].w, segments[i].s, x, yi, workspace, workspace_bytes, bf16, pdl, 0, cs,
                                static_cast<int>(total), (flags & MATGPTQ_B200_FLAG_SCRATCH_REDUCE) != 0);
       else
         r = mg::gemv_launch(static_cast<int>(segments[i].bitwidth), static_cast<int>(group_size),
@@ -325,10 +325,7 @@ int matgptq_b200_device_status(int *status_out, int reset) {
   int e = 0;
   r = mg::selftest_device_status(&e, reset);
   if (r != MG_OK) return r;
-  int f = 0;
-  r = mg::gemm_tc_zp_device_status(&f, reset);
-  if (r != MG_OK) return r;
-  if (status_out) *status_out = a ? a : (b ? b : (d ? d : (e ? e : f)));
+  if (status_out) *status_out = a ? a : (b ? b : (d ? d : e));
   return MG_OK;
 }
 

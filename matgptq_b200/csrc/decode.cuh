@@ -272,19 +272,6 @@ template <int B> __device__ __forceinline__ uint32_t dense_int_bf16(const uint32
   }
 }
 
-// Pair P of a lane as half2 integers (code - Z) * DensePre<B>.
-template <int B> __device__ __forceinline__ uint32_t dense_int_f16(const uint32_t (&w)[2 * B], int P) {
-  const uint32_t x = field_pair<B>(w, P, kMagic);
-  switch (kstep_offset<B>(P >> 2)) {  // a compile-time constant once the caller's loops are unrolled
-    case 0: return dense_int_at<B, 0>(x);
-    case 2: return dense_int_at<B, 2>(x);
-    case 3: return dense_int_at<B, 3>(x);
-    case 4: return dense_int_at<B, 4>(x);
-    case 6: return dense_int_at<B, 6>(x);
-    default: return dense_int_at<B, 8>(x);
-  }
-}
-
 // scale2: dense_scale() of the row's scale
 template <int B, bool BF16>
 __device__ __forceinline__ uint32_t dense_pair(const uint32_t (&w)[2 * B], int P, uint32_t scale2) {
@@ -293,37 +280,17 @@ __device__ __forceinline__ uint32_t dense_pair(const uint32_t (&w)[2 * B], int P
     const __nv_bfloat162 r = __hmul2(*reinterpret_cast<const __nv_bfloat162 *>(&scale2), *reinterpret_cast<const __nv_bfloat162 *>(&vb));
     return *reinterpret_cast<const uint32_t *>(&r);
   }
-  return h2_bits(__hmul2(bits_h2(scale2), bits_h2(dense_int_f16<B>(w, P))));
-}
-
-// The same with a zero point of its own: s * (code * 2^(8-b) - zero), bit for bit what dequant_pair() gives with
-// has_zero.  The exact integer (code - Z) * DensePre becomes (code - Z) * 2^(8-b) + (128 - zero) in one more
-// instruction (an addition, or the fma that also takes the rest of 2^(8-b)), exact for every zero point of a master
-// byte.  scale2: the scale in both halves (not dense_scale()); off2: dense_zero() of the zero point.
-template <bool BF16> __device__ __forceinline__ uint32_t dense_zero(uint16_t zero) {
-  const uint32_t zb = splat16(zero);
-  if constexpr (BF16) {
-    const __nv_bfloat162 r = __hsub2(__float2bfloat162_rn(128.f), *reinterpret_cast<const __nv_bfloat162 *>(&zb));
-    return *reinterpret_cast<const uint32_t *>(&r);
-  } else {
-    return h2_bits(__hsub2(__float2half2_rn(128.f), bits_h2(zb)));
+  const uint32_t x = field_pair<B>(w, P, kMagic);
+  uint32_t v;
+  switch (kstep_offset<B>(P >> 2)) {  // a compile-time constant once the caller's loops are unrolled
+    case 0: v = dense_int_at<B, 0>(x); break;
+    case 2: v = dense_int_at<B, 2>(x); break;
+    case 3: v = dense_int_at<B, 3>(x); break;
+    case 4: v = dense_int_at<B, 4>(x); break;
+    case 6: v = dense_int_at<B, 6>(x); break;
+    default: v = dense_int_at<B, 8>(x); break;
   }
-}
-
-template <int B, bool BF16>
-__device__ __forceinline__ uint32_t dense_pair_zero(const uint32_t (&w)[2 * B], int P, uint32_t scale2, uint32_t off2) {
-  constexpr float rest = static_cast<float>((1 << (8 - B)) / DensePre<B>::value);
-  if constexpr (BF16) {
-    const uint32_t vb = dense_int_bf16<B>(w, P);
-    const __nv_bfloat162 v = *reinterpret_cast<const __nv_bfloat162 *>(&vb), o = *reinterpret_cast<const __nv_bfloat162 *>(&off2);
-    const __nv_bfloat162 q = (rest == 1.f) ? __hadd2(v, o) : __hfma2(v, __float2bfloat162_rn(rest), o);
-    const __nv_bfloat162 r = __hmul2(*reinterpret_cast<const __nv_bfloat162 *>(&scale2), q);
-    return *reinterpret_cast<const uint32_t *>(&r);
-  } else {
-    const __half2 v = bits_h2(dense_int_f16<B>(w, P)), o = bits_h2(off2);
-    const __half2 q = (rest == 1.f) ? __hadd2(v, o) : __hfma2(v, __float2half2_rn(rest), o);
-    return h2_bits(__hmul2(bits_h2(scale2), q));
-  }
+  return h2_bits(__hmul2(bits_h2(scale2), bits_h2(v)));
 }
 
 // Coalesced load of a lane's words of one block (all lanes of a warp call it).

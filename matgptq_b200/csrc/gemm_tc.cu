@@ -31,16 +31,7 @@
 #include "host_util.h"
 #include "kernels.h"
 
-// This file is compiled twice: as it is (implicit zero point 2^(b-1), what the reference's operator computes) and from
-// gemm_tc_zp.cu with MG_TC_ZP = 1 (per-group zero points, an extension).  Everything that differs between the two
-// carries kZP in its template arguments or its name, so the two objects link together.
-#ifndef MG_TC_ZP
-#define MG_TC_ZP 0
-#endif
-
 namespace mg {
-
-constexpr bool kZP = MG_TC_ZP != 0;
 
 // A pipeline stage covers 64 in-features (half a packed block).
 constexpr int kTcChunkStride = 2080;   // bytes between 16-byte K chunks of the A stage: 128 rows * 16 B + 32 B
@@ -50,7 +41,6 @@ constexpr int kTcAStageBytes = 8 * kTcChunkStride;  // 8 chunks of 8 in-features
 struct GemmParams {
   const uint32_t *w;
   const uint16_t *s;
-  const uint16_t *z;  // zero points in master units, laid out like the scales (only read when kZP)
   const uint16_t *x;
   uint16_t *y;
   int N, K, M;
@@ -189,61 +179,32 @@ template <int OFF> __device__ __forceinline__ void sts_v4(uint32_t addr, const u
                : "memory");
 }
 
-// What a lane needs of one scale group to make dense weights of rows g (lo) and g+8 (hi)
-struct TcGroup {
-  uint32_t s_lo, s_hi;  // scales in both halves (dense_scale() without zero points)
-  uint32_t z_lo, z_hi;  // dense_zero() of the zero points (kZP)
-};
-
-// raw scales (and zero points) of rows g and g+8 for the groups of a block
-template <int GS> struct TcRaw {
-  uint16_t s_lo[TcScales<GS>::NG], s_hi[TcScales<GS>::NG];
-  uint16_t z_lo[kZP ? TcScales<GS>::NG : 1], z_hi[kZP ? TcScales<GS>::NG : 1];
-};
-
-template <int B, int GS, bool BF16> __device__ __forceinline__ TcGroup tc_group(const TcRaw<GS> &r, int i) {
-  TcGroup g;
-  if constexpr (kZP) {
-    g.s_lo = splat16(r.s_lo[i]);
-    g.s_hi = splat16(r.s_hi[i]);
-    g.z_lo = dense_zero<BF16>(r.z_lo[i]);
-    g.z_hi = dense_zero<BF16>(r.z_hi[i]);
-  } else {
-    g.s_lo = dense_scale<B, BF16>(r.s_lo[i]);
-    g.s_hi = dense_scale<B, BF16>(r.s_hi[i]);
-    g.z_lo = g.z_hi = 0u;
-  }
-  return g;
-}
-
-template <int B, bool BF16> __device__ __forceinline__ uint32_t tc_pair(const uint32_t (&w)[2 * B], int P, uint32_t s, uint32_t z) {
-  return kZP ? dense_pair_zero<B, BF16>(w, P, s, z) : dense_pair<B, BF16>(w, P, s);
-}
-
 // Chunk JJ (0..3, 32 in-features) of a block: this lane's dense weights of rows g (lo) and g+8 (hi), eight each, as
 // 16 bytes per row into the A tile whose lane address for chunk 0 is `addr`.
 template <int B, bool BF16, int JJ>
-__device__ __forceinline__ void tc_store_chunk(const uint32_t (&w)[2 * B], const TcGroup &g, uint32_t addr) {
+__device__ __forceinline__ void tc_store_chunk(const uint32_t (&w)[2 * B], uint32_t s_lo, uint32_t s_hi, uint32_t addr) {
   uint4 lo, hi;
-  lo.x = tc_pair<B, BF16>(w, 8 * JJ + 0, g.s_lo, g.z_lo);
-  lo.y = tc_pair<B, BF16>(w, 8 * JJ + 2, g.s_lo, g.z_lo);
-  lo.z = tc_pair<B, BF16>(w, 8 * JJ + 4, g.s_lo, g.z_lo);
-  lo.w = tc_pair<B, BF16>(w, 8 * JJ + 6, g.s_lo, g.z_lo);
-  hi.x = tc_pair<B, BF16>(w, 8 * JJ + 1, g.s_hi, g.z_hi);
-  hi.y = tc_pair<B, BF16>(w, 8 * JJ + 3, g.s_hi, g.z_hi);
-  hi.z = tc_pair<B, BF16>(w, 8 * JJ + 5, g.s_hi, g.z_hi);
-  hi.w = tc_pair<B, BF16>(w, 8 * JJ + 7, g.s_hi, g.z_hi);
+  lo.x = dense_pair<B, BF16>(w, 8 * JJ + 0, s_lo);
+  lo.y = dense_pair<B, BF16>(w, 8 * JJ + 2, s_lo);
+  lo.z = dense_pair<B, BF16>(w, 8 * JJ + 4, s_lo);
+  lo.w = dense_pair<B, BF16>(w, 8 * JJ + 6, s_lo);
+  hi.x = dense_pair<B, BF16>(w, 8 * JJ + 1, s_hi);
+  hi.y = dense_pair<B, BF16>(w, 8 * JJ + 3, s_hi);
+  hi.z = dense_pair<B, BF16>(w, 8 * JJ + 5, s_hi);
+  hi.w = dense_pair<B, BF16>(w, 8 * JJ + 7, s_hi);
   sts_v4<(JJ & 1) * 4 * kTcChunkStride>(addr, lo);
   sts_v4<(JJ & 1) * 4 * kTcChunkStride + 128>(addr, hi);
 }
 
-// Half H (0, 1) of a block = chunks 2H and 2H+1 = one pipeline stage
+// Half H (0, 1) of a block = chunks 2H and 2H+1 = one pipeline stage; slo/shi: raw scales of rows g and g+8
 template <int B, int GS, bool BF16, int H>
-__device__ __forceinline__ void tc_store_half(const uint32_t (&w)[2 * B], const TcRaw<GS> &raw, uint32_t addr) {
+__device__ __forceinline__ void tc_store_half(const uint32_t (&w)[2 * B], const uint16_t (&slo)[TcScales<GS>::NG],
+                                              const uint16_t (&shi)[TcScales<GS>::NG], uint32_t addr) {
   constexpr int g0 = (GS == 32) ? 2 * H : 0, g1 = (GS == 32) ? 2 * H + 1 : 0;
-  const TcGroup a = tc_group<B, GS, BF16>(raw, g0);
-  tc_store_chunk<B, BF16, 2 * H>(w, a, addr);
-  tc_store_chunk<B, BF16, 2 * H + 1>(w, (GS == 32) ? tc_group<B, GS, BF16>(raw, g1) : a, addr);
+  const uint32_t lo0 = dense_scale<B, BF16>(slo[g0]), hi0 = dense_scale<B, BF16>(shi[g0]);
+  tc_store_chunk<B, BF16, 2 * H>(w, lo0, hi0, addr);
+  const uint32_t lo1 = (GS == 32) ? dense_scale<B, BF16>(slo[g1]) : lo0, hi1 = (GS == 32) ? dense_scale<B, BF16>(shi[g1]) : hi0;
+  tc_store_chunk<B, BF16, 2 * H + 1>(w, lo1, hi1, addr);
 }
 
 struct TcProducer {
@@ -256,10 +217,11 @@ struct TcProducer {
 // over, move on to the next stage.  `mine` false: the half belongs to the other warp of the pair.
 template <int B, int GS, bool BF16, int H>
 __device__ __forceinline__ bool tc_producer_half(TcProducer &pr, bool mine, bool valid, int lane, const uint32_t (&w)[2 * B],
-                                                 const TcRaw<GS> &raw) {
+                                                 const uint16_t (&slo)[TcScales<GS>::NG],
+                                                 const uint16_t (&shi)[TcScales<GS>::NG]) {
   if (mine) {
     if (!mbar_wait(pr.bar_empty + pr.idx8, pr.parity)) return false;  // the tensor pipe is done with what this stage held
-    if (valid) tc_store_half<B, GS, BF16, H>(w, raw, pr.a_lane + pr.off);
+    if (valid) tc_store_half<B, GS, BF16, H>(w, slo, shi, pr.a_lane + pr.off);
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic-proxy stores -> tensor pipe reads
     __syncwarp();
     if (lane == 0) mbar_arrive(pr.bar_full + pr.idx8);
@@ -341,33 +303,24 @@ __device__ __forceinline__ void gemm_tc_body(const GemmParams &p, const CUtensor
     // modulo by the (runtime) number of stages.
     constexpr int kAhead = (B >= 6) ? 3 : (PW == 16 ? 4 : 6);
     const uint32_t *wnext = p.w + (static_cast<size_t>(valid ? tile16 : 0) * p.kblocks + kb_lo) * BW;  // next block to load
-    const size_t s_first = (static_cast<size_t>(valid ? tile16 : 0) * groups + ((GS == -1) ? 0 : kb_lo * NG)) * 16 + g;
-    const uint16_t *snext = p.s + s_first;
-    const uint16_t *znext = kZP ? p.z + s_first : nullptr;
+    const uint16_t *snext = p.s + (static_cast<size_t>(valid ? tile16 : 0) * groups + ((GS == -1) ? 0 : kb_lo * NG)) * 16 + g;
     uint32_t wq[kAhead][2 * B];
     // raw scales of rows g and g+8, loaded with the block's words and only touched when the block is decoded
     // (dense_scale() applied on arrival would stall the warp on the load it has just issued)
-    TcRaw<GS> sq[kAhead];
-    auto load_next = [&](uint32_t (&wdst)[2 * B], TcRaw<GS> &raw) {
+    uint16_t sq_lo[kAhead][NG], sq_hi[kAhead][NG];
+    auto load_next = [&](uint32_t (&wdst)[2 * B], uint16_t (&lo)[NG], uint16_t (&hi)[NG]) {
       load_block<B>(wnext, lane, wdst);
 #pragma unroll
       for (int j = 0; j < NG; ++j) {
-        raw.s_lo[j] = ldg_u16_tc(snext + j * 16);
-        raw.s_hi[j] = ldg_u16_tc(snext + j * 16 + 8);
-        if constexpr (kZP) {
-          raw.z_lo[j] = ldg_u16_tc(znext + j * 16);
-          raw.z_hi[j] = ldg_u16_tc(znext + j * 16 + 8);
-        }
+        lo[j] = ldg_u16_tc(snext + j * 16);
+        hi[j] = ldg_u16_tc(snext + j * 16 + 8);
       }
       wnext += BW;
-      if (GS != -1) {
-        snext += NG * 16;
-        if (kZP) znext += NG * 16;
-      }
+      if (GS != -1) snext += NG * 16;
     };
 #pragma unroll
     for (int a = 0; a < kAhead; ++a)
-      if (valid && a < nblk) load_next(wq[a], sq[a]);
+      if (valid && a < nblk) load_next(wq[a], sq_lo[a], sq_hi[a]);
 
     // this lane's 16 bytes of rows g and g+8 in the A tile of stage 0, chunk t (shared-memory address)
     const uint32_t a_lane = base_u32 + plan.off_stages + plan.b_stage_bytes + t * kTcChunkStride + (2 * ptile) * 128 + g * 16;
@@ -385,11 +338,11 @@ __device__ __forceinline__ void gemm_tc_body(const GemmParams &p, const CUtensor
 #pragma unroll
       for (int a = 0; a < kAhead; ++a) {
         if (blk + a < nblk && !failed) {
-          if (!tc_producer_half<B, GS, BF16, 0>(pr, PW == 8 || my_half == 0, valid, lane, wq[a], sq[a]) ||
-              !tc_producer_half<B, GS, BF16, 1>(pr, PW == 8 || my_half == 1, valid, lane, wq[a], sq[a])) {
+          if (!tc_producer_half<B, GS, BF16, 0>(pr, PW == 8 || my_half == 0, valid, lane, wq[a], sq_lo[a], sq_hi[a]) ||
+              !tc_producer_half<B, GS, BF16, 1>(pr, PW == 8 || my_half == 1, valid, lane, wq[a], sq_lo[a], sq_hi[a])) {
             failed = true;
           } else if (valid && blk + a + kAhead < nblk) {
-            load_next(wq[a], sq[a]);  // this block's registers are free: fetch the block kAhead ahead
+            load_next(wq[a], sq_lo[a], sq_hi[a]);  // this block's registers are free: fetch the block kAhead ahead
           }
         }
       }
@@ -550,14 +503,14 @@ __device__ __forceinline__ void gemm_tc_body(const GemmParams &p, const CUtensor
   }
 }
 
-template <int B, int GS, bool BF16, int PW, bool ZP>
+template <int B, int GS, bool BF16, int PW>
 __global__ void __launch_bounds__((PW + 2) * 32, PW == 8 ? 2 : 1) gemm_tc_kernel(const GemmParams p, const __grid_constant__ CUtensorMap xmap) {
   gemm_tc_body<B, GS, BF16, PW>(p, xmap, static_cast<int>(blockIdx.x));
 }
 
 // partial[split][M][N] fp32 -> y[M][N] (rows ldy elements apart), added in the order of the K ranges: the second
 // kernel of a K split that goes through scratch memory
-template <bool BF16, bool ZP>
+template <bool BF16>
 __global__ void splitk_reduce_kernel(const float *__restrict__ partial, uint16_t *__restrict__ y, long long mn, int split,
                                      int n_cols, int ldy) {
   // launched with programmatic stream serialization right behind the kernel that writes `partial`
@@ -585,7 +538,7 @@ constexpr int kTcHalfSmBytes = 112 * 1024;
 static bool tc_two_ctas_per_sm(int ncols) { return tc_plan(ncols, 3).total <= kTcHalfSmBytes; }
 
 // K split of the tensor-core path: one wave of CTAs over the SMs' slots; at least four blocks of K per CTA.
-static int pick_split(int N, int K, int M, int sm_count) {
+int gemm_tc_pick_split(int N, int K, int M, int sm_count) {
   const int ctas = ((N + 127) / 128) * ((M + 255) / 256);
   const int kblocks = K / 128;
   const int want = tc_two_ctas_per_sm(round_up16(M < 256 ? M : 256)) ? 2 * sm_count : sm_count;
@@ -594,21 +547,11 @@ static int pick_split(int N, int K, int M, int sm_count) {
   return split;
 }
 
-#if MG_TC_ZP
-#define MG_TC_LAUNCH gemm_tc_zp_launch
-#define MG_TC_STATUS gemm_tc_zp_device_status
-#else
-#define MG_TC_LAUNCH gemm_tc_launch
-#define MG_TC_STATUS gemm_tc_device_status
-
-int gemm_tc_pick_split(int N, int K, int M, int sm_count) { return pick_split(N, K, M, sm_count); }
-
 // Scratch for a K split that goes through global memory (scratch_reduce, or a device that cannot place the cluster).
 long long gemm_tc_workspace_bytes(int N, int K, int M, int sm_count) {
-  const int split = pick_split(N, K, M, sm_count);
+  const int split = gemm_tc_pick_split(N, K, M, sm_count);
   return split > 1 ? static_cast<long long>(split) * M * N * 4 : 0;
 }
-#endif
 
 // Tensor map of the activations x[M, K] (two-byte elements, row-major) with boxes of 64 in-features x `box_rows`
 // batch rows and the 128-byte swizzle the UMMA descriptor of the B operand expects; rows past M read as zeros.
@@ -648,7 +591,7 @@ static int tc_pick_stages(int ncols, int producer_warps) {
 
 template <int B, int GS, bool BF16, int PW>
 static int launch_gemm_tc_warps(GemmParams p, cudaStream_t stream, bool pdl, float *fallback_partial) {
-  auto kernel = gemm_tc_kernel<B, GS, BF16, PW, kZP>;
+  auto kernel = gemm_tc_kernel<B, GS, BF16, PW>;
   CUtensorMap xmap;
   if (make_x_tensor_map(&xmap, p.x, p.M, p.K, p.ncols) != MG_OK) return MG_ERR_CUDA;
   const int stages = tc_pick_stages(p.ncols, PW);
@@ -704,7 +647,7 @@ static int launch_gemm_tc_warps(GemmParams p, cudaStream_t stream, bool pdl, flo
     rattr[0].val.programmaticStreamSerializationAllowed = 1;
     rcfg.attrs = rattr;
     rcfg.numAttrs = 1;
-    if (cudaLaunchKernelEx(&rcfg, splitk_reduce_kernel<BF16, kZP>, static_cast<const float *>(p.partial), p.y, mn, p.split, p.N, p.ldy) != cudaSuccess)
+    if (cudaLaunchKernelEx(&rcfg, splitk_reduce_kernel<BF16>, static_cast<const float *>(p.partial), p.y, mn, p.split, p.N, p.ldy) != cudaSuccess)
       return MG_ERR_CUDA;
   }
   return MG_OK;
@@ -746,11 +689,9 @@ static int launch_gemm_tc_group(const GemmParams &p, int group_size, bool bf16, 
 
 // workspace: fp32 scratch of at least gemm_tc_workspace_bytes() or null.  The sums of a split K meet inside a
 // thread-block cluster; the scratch is used when scratch_reduce asks for it, or when the cluster cannot be launched.
-// z: zero points (reordered like the scales) for the build with zero points, null for the other one.
-int MG_TC_LAUNCH(int bitwidth, int group_size, int N, int K, int M, const void *w, const void *s, const void *z, const void *x,
+int gemm_tc_launch(int bitwidth, int group_size, int N, int K, int M, const void *w, const void *s, const void *x,
                    void *y, void *workspace, long long workspace_bytes, bool bf16, bool pdl, int split_override,
                    cudaStream_t stream, int ldy, bool scratch_reduce) {
-  if (kZP != (z != nullptr)) return MG_ERR_BAD_ARG;
   int sm_count = 0;  // of the current device
   {
     const int st = current_device_sm_count(&sm_count);
@@ -759,7 +700,6 @@ int MG_TC_LAUNCH(int bitwidth, int group_size, int N, int K, int M, const void *
   GemmParams p;
   p.w = static_cast<const uint32_t *>(w);
   p.s = static_cast<const uint16_t *>(s);
-  p.z = static_cast<const uint16_t *>(z);
   p.x = static_cast<const uint16_t *>(x);
   p.y = static_cast<uint16_t *>(y);
   p.N = N;
@@ -767,7 +707,7 @@ int MG_TC_LAUNCH(int bitwidth, int group_size, int N, int K, int M, const void *
   p.M = M;
   p.ldy = ldy > 0 ? ldy : N;
   p.kblocks = K / 128;
-  int split = split_override > 0 ? split_override : pick_split(N, K, M, sm_count);
+  int split = split_override > 0 ? split_override : gemm_tc_pick_split(N, K, M, sm_count);
   if (split > p.kblocks) split = p.kblocks;
   if (split > 8) return MG_ERR_BAD_ARG;  // the CTAs along K form one cluster
   const bool have_scratch = workspace != nullptr && workspace_bytes >= static_cast<long long>(split) * M * N * 4;
@@ -787,6 +727,6 @@ int MG_TC_LAUNCH(int bitwidth, int group_size, int N, int K, int M, const void *
   }
 }
 
-MG_DEFINE_STATUS_ACCESSOR(MG_TC_STATUS)
+MG_DEFINE_STATUS_ACCESSOR(gemm_tc_device_status)
 
 }  // namespace mg

@@ -59,15 +59,10 @@ int gemv_zp_device_status(int *status_out, int reset);
 // gemm_tc.cu
 int gemm_tc_pick_split(int N, int K, int M, int sm_count);
 long long gemm_tc_workspace_bytes(int N, int K, int M, int sm_count);
-// z must be null for gemm_tc_launch and non-null for gemm_tc_zp_launch (gemm_tc_zp.cu: the same kernels with zero points)
-int gemm_tc_launch(int bitwidth, int group_size, int N, int K, int M, const void *w, const void *s, const void *z,
-                   const void *x, void *y, void *workspace, long long workspace_bytes, bool bf16, bool pdl,
-                   int split_override, cudaStream_t stream, int ldy = 0, bool scratch_reduce = false);
-int gemm_tc_zp_launch(int bitwidth, int group_size, int N, int K, int M, const void *w, const void *s, const void *z,
-                      const void *x, void *y, void *workspace, long long workspace_bytes, bool bf16, bool pdl,
-                      int split_override, cudaStream_t stream, int ldy = 0, bool scratch_reduce = false);
+int gemm_tc_launch(int bitwidth, int group_size, int N, int K, int M, const void *w, const void *s, const void *x,
+                   void *y, void *workspace, long long workspace_bytes, bool bf16, bool pdl, int split_override,
+                   cudaStream_t stream, int ldy = 0, bool scratch_reduce = false);
 int gemm_tc_device_status(int *status_out, int reset);
-int gemm_tc_zp_device_status(int *status_out, int reset);
 
 // selftest.cu
 int selftest_device_status(int *status_out, int reset);
