@@ -122,9 +122,18 @@ Tensor reorder(const Tensor &scales, int64_t m, int64_t n, int64_t group_size) {
 
 Tensor dequantize(const Tensor &weights, const Tensor &scales, int64_t n_out, int64_t n_in, int64_t bitwidth, int64_t group_size,
                   int64_t flags) {
+  // the C ABI sees addresses only: what the kernel reads has to be on the GPU, dense and as large as the shape says
+  TORCH_CHECK(weights.is_cuda(), "dequantize_matgptq: expected matgptq_weights to be a CUDA tensor");
+  TORCH_CHECK(scales.is_cuda() && scales.device() == weights.device(),
+              "dequantize_matgptq: expected matgptq_scales to be a CUDA tensor on the GPU of matgptq_weights");
   check_common(bitwidth, group_size, n_in);
   TORCH_CHECK(scales.scalar_type() == type_of(flags), "matgptq_scales must be ", type_name(flags), " for feature_flag=", flags);
-  const c10::Device dev = cuda_device_of(weights);
+  const int64_t groups = group_size == -1 ? 1 : n_in / group_size;
+  TORCH_CHECK(weights.is_contiguous() && weights.element_size() == 4 && weights.numel() >= bitwidth * n_out * n_in / 32,
+              "matgptq_weights must hold ", bitwidth * n_out * n_in / 32, " contiguous 32-bit words");
+  TORCH_CHECK(scales.is_contiguous() && scales.numel() >= n_out * groups, "matgptq_scales must hold ", n_out * groups,
+              " contiguous elements");
+  const c10::Device dev = weights.device();
   const c10::cuda::CUDAGuard on_device(dev);
   Tensor out = empty_on({n_out, n_in}, type_of(flags), dev);
   check_status(lib.dequantize(static_cast<const uint32_t *>(weights.const_data_ptr()), scales.const_data_ptr(), nullptr, out.data_ptr(),
@@ -296,8 +305,8 @@ TORCH_LIBRARY(matgptq_cuda, m) {
         "SymInt bitwidth, SymInt group_size, SymInt feature_flag) -> Tensor", tags);
 }
 
-// The CPU registrations move what the load-time operators may take from the host, and say for the others that there
-// is no CPU implementation.
+// The CPU registrations move what the packers and the reordering take from the host; the other operators refuse host
+// tensors there.
 #define MG_REGISTER(key)                                                    \
   TORCH_LIBRARY_IMPL(matgptq_cuda, key, m) {                                \
     m.impl("pack_matgptq_qweights", pack);                                  \
