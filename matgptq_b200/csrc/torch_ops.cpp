@@ -336,10 +336,14 @@ struct WithoutGil {  // a launch may wait for room in the stream's queue: other 
   ~WithoutGil() { PyEval_RestoreThread(state); }
 };
 
+// A tensor whose bytes are what the kernel would read.  The keys are those of an ordinary CUDA tensor and nothing else: one
+// with the negative bit or without storage, or a subclass's, has a key of its own and is the dispatcher's to materialise.
 bool plain_cuda(PyObject *o) {
   if (!THPVariable_CheckExact(o)) return false;
   const Tensor &t = THPVariable_Unpack(o);
-  return t.is_cuda() && t.layout() == at::kStrided && !t.key_set().has(c10::DispatchKey::Python);
+  constexpr c10::DispatchKeySet ordinary({c10::DispatchKey::CUDA, c10::DispatchKey::AutogradCUDA, c10::DispatchKey::ADInplaceOrView,
+                                          c10::DispatchKey::AutocastCUDA});
+  return t.is_cuda() && t.layout() == at::kStrided && (t.key_set() - ordinary).highestFunctionalityKey() == c10::DispatchKey::Undefined;
 }
 
 // nothing between the caller and the kernel wants to see the call

@@ -54,3 +54,55 @@ def test_bad_inputs_raise(cuda):
                 torch.randn(3, 256, dtype=torch.float16)):
         with pytest.raises(RuntimeError):
             layer(bad)
+
+
+def _direct(layer, x):
+    from matgptq_b200 import ops
+    return ops._ext.linear_forward(x, layer.matgptq_qweight, layer.matgptq_scales, layer.n_out_features, layer.n_in_features,
+                                   layer.bitwidth, layer.group_size, 1)
+
+
+@pytest.mark.gpu
+def test_ordinary_tensors_take_the_direct_path(cuda):
+    layer = _layer(cuda)
+    k = layer.n_in_features
+    base = torch.randn(12, 2 * k + 8, dtype=torch.float16, device=cuda)
+    grad = base[:, :k].contiguous().requires_grad_()
+    with torch.inference_mode():
+        inference = base[:, :k] + 0
+    for x in (base[:, :k].contiguous(), base[:, k:2 * k], base.flatten()[1:1 + 12 * k].view(3, 4, k), base[:0, :k], grad,
+              torch.nn.Parameter(base[:, :k].contiguous()), inference):
+        y = _direct(layer, x)
+        assert y is not None and torch.equal(y.view(-1, layer.n_out_features), _op(layer, x.detach().reshape(-1, k).clone()))
+
+    class Seen(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            return func(*args, **(kwargs or {}))
+
+    with Seen():
+        assert _direct(layer, base[:, :k].contiguous()) is None
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("form", ["negative_bit", "conjugate_imag", "zero_tensor", "subclass"])
+def test_tensors_that_are_not_their_storage_take_the_operator(cuda, form):
+    layer = _layer(cuda)
+    shape = (4, layer.n_in_features)
+    values = torch.randn(shape, dtype=torch.float16, device=cuda)
+
+    class Sub(torch.Tensor):
+        pass
+
+    if form == "negative_bit":
+        x, same = torch._neg_view(values), -values
+    elif form == "conjugate_imag":  # a plain way to the same bit
+        x = torch.view_as_complex(torch.stack([values, values], -1)).conj().imag
+        same = -values
+    elif form == "zero_tensor":
+        x = torch._efficientzerotensor(shape, dtype=torch.float16, device=cuda)
+    else:
+        x, same = values.as_subclass(Sub), values
+    assert _direct(layer, x) is None
+    if form != "zero_tensor":  # it has no memory at all; the operator says what it thinks of that
+        y = layer(x)
+        assert torch.equal(torch.Tensor(y) if form == "subclass" else y, _op(layer, same))
