@@ -21,7 +21,9 @@
 #include <c10/cuda/CUDAStream.h>
 #include <dlfcn.h>
 #include <torch/csrc/Exceptions.h>
-#include <torch/csrc/autograd/autograd_not_implemented_fallback.h>
+#include <torch/csrc/autograd/VariableTypeUtils.h>
+#include <torch/csrc/autograd/functions/basic_ops.h>
+#include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/library.h>
 
@@ -222,7 +224,6 @@ void matmul_out(const Tensor &input, const Tensor &weights, const Tensor &scales
   const Tensor x = prepare_input(input, batch, n_in);
   launch_matmul("matmul_matgptq_out", dev, bitwidth, group_size, n_out, n_in, batch, weights, scales, x.const_data_ptr(), out.data_ptr(),
                 flags);
-  if (!out.is_inference()) out.unsafeGetTensorImpl()->bump_version();
 }
 
 // The C-ABI grouped product: segment i fills its column block of out [M, sum(n_out)].
@@ -321,11 +322,59 @@ TORCH_LIBRARY(matgptq_cuda, m) {
 MG_REGISTER(CPU)
 MG_REGISTER(CUDA)
 
-// No operator has a derivative: results of inputs that require one say so when backward reaches them.
+// ---- autograd -------------------------------------------------------------------------------------------------
+namespace {
+
+// No operator has a derivative: a result of inputs that require one says so when backward reaches it.  Any other call goes
+// on below autograd as it is; forward-mode tangents end here, and `out` may be a leaf that requires a gradient.
+void without_derivative(const c10::OperatorHandle &op, c10::DispatchKeySet keys, torch::jit::Stack *stack) {
+  std::vector<Tensor> inputs;  // those that require a gradient
+  const auto &arguments = op.schema().arguments();
+  if (at::GradMode::is_enabled()) {
+    const size_t first = stack->size() - arguments.size();
+    const auto add = [&](const Tensor &t) {
+      if (!t.requires_grad()) return;
+      TORCH_CHECK_NOT_IMPLEMENTED(!torch::autograd::isFwGradDefined(t), "forward AD through ", op.schema().name(), " is not implemented");
+      inputs.push_back(t);
+    };
+    for (size_t i = 0; i < arguments.size(); ++i) {
+      const c10::IValue &v = (*stack)[first + i];
+      if (arguments[i].alias_info()) continue;  // written, not read
+      if (v.isTensor()) add(v.toTensor());
+      if (v.isTensorList())
+        for (const Tensor &t : v.toTensorVector()) add(t);
+    }
+  }
+  {
+    const at::AutoDispatchBelowAutograd below;
+    op.redispatchBoxed(keys & c10::after_autograd_keyset, stack);
+  }
+  if (inputs.empty() || op.schema().returns().empty()) return;
+  const auto node = std::make_shared<torch::autograd::NotImplemented>(op.schema().name(), torch::autograd::collect_next_edges(inputs));
+  Tensor result = stack->back().toTensor();
+  torch::autograd::set_history(result, node);
+}
+
+// matmul_matgptq_out writes its last argument
+void counts_as_write(const c10::OperatorHandle &op, c10::DispatchKeySet keys, torch::jit::Stack *stack) {
+  const Tensor out = stack->back().toTensor();
+  {
+    const at::AutoDispatchBelowADInplaceOrView below;
+    op.redispatchBoxed(keys & c10::after_ADInplaceOrView_keyset, stack);
+  }
+  if (!out.is_inference()) out.unsafeGetTensorImpl()->bump_version();
+}
+
+}  // namespace
+
 TORCH_LIBRARY_IMPL(matgptq_cuda, Autograd, m) {
   for (const char *name : {"pack_matgptq_qweights", "slice_pack_matgptq_qweights", "reorder_matgptq_scales", "matmul_matgptq",
                            "matmul_matgptq_out", "matmul_matgptq_grouped", "matmul_matgptq_zeros", "dequantize_matgptq"})
-    m.impl(name, torch::autograd::autogradNotImplementedFallback());
+    m.impl(name, torch::CppFunction::makeFromBoxedFunction<&without_derivative>());
+}
+
+TORCH_LIBRARY_IMPL(matgptq_cuda, ADInplaceOrView, m) {
+  m.impl("matmul_matgptq_out", torch::CppFunction::makeFromBoxedFunction<&counts_as_write>());
 }
 
 // ---- Python module --------------------------------------------------------------------------------------------
