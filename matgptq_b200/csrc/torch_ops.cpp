@@ -406,9 +406,9 @@ bool dispatcher_not_needed() {
          at::impl::PythonTorchFunctionTLS::stack_len() == 0 && c10::impl::PythonDispatcherTLS::get_state() == nullptr;
 }
 
+// Whole numbers, numpy's among them (anything with __index__).
 bool as_ints(PyObject *const *args, Py_ssize_t n, int64_t *out) {
   for (Py_ssize_t i = 0; i < n; ++i) {
-    if (!PyLong_Check(args[i])) return false;
     out[i] = PyLong_AsLongLong(args[i]);
     if (out[i] == -1 && PyErr_Occurred()) {
       PyErr_Clear();

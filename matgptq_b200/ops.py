@@ -96,7 +96,8 @@ def matmul_matgptq_grouped_raw(x: torch.Tensor, packed, scales, n_out, n_in: int
     """The C-ABI grouped product without checks: segment ``i`` (``packed[i]``, ``scales[i]``, ``n_out[i]`` rows at
     ``bitwidths[i]`` bits) fills its column block of ``out [M, sum(n_out)]``.  One kernel launch up to 16 rows."""
     if out is None and workspace is None:
-        return _ext.grouped_raw(x, list(packed), list(scales), list(n_out), n_in, list(bitwidths), group_size, flags)
+        return _ext.grouped_raw(x, list(packed), list(scales), [int(n) for n in n_out], n_in, [int(b) for b in bitwidths],
+                                group_size, flags)
     batch = x.size(-2)
     total = int(sum(n_out))
     if out is None:

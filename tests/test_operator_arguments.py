@@ -1,4 +1,5 @@
 """What the operators refuse before anything is launched, and what autograd makes of them."""
+import numpy as np
 import pytest
 import torch
 import torch.autograd.forward_ad as forward_ad
@@ -87,3 +88,18 @@ def test_a_tangent_does_not_change_where_a_call_fails():
     scales = torch.ones(N, 3, dtype=torch.float16)
     with forward_ad.dual_level(), pytest.raises(RuntimeError, match="scales must have shape"):
         torch.ops.matgptq_cuda.reorder_matgptq_scales(forward_ad.make_dual(scales, torch.ones_like(scales)), N, K, G)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("number", [np.int64, np.int32, torch.tensor])
+def test_raw_entries_take_any_whole_number(cuda, number):
+    words, scales = _tensors(cuda)
+    x = torch.randn(2, K, dtype=torch.float16, device=cuda)
+    want = _matmul(x, words, scales)
+    assert torch.equal(ops.matmul_matgptq_raw(x, words, scales, *(number(v) for v in (N, K, B, G, 1))), want)
+    assert torch.equal(ops.matmul_matgptq_grouped_raw(x, (words,), (scales,), (number(N),), number(K), (number(B),), number(G), number(1)),
+                       want)
+    if number is not torch.tensor:
+        assert torch.equal(ops.matmul_matgptq_grouped_raw(x, [words], [scales], np.array([N]), K, np.array([B], dtype=np.uint8), G, 1), want)
+    with pytest.raises(RuntimeError):
+        ops.matmul_matgptq_raw(x, words, scales, float(N), K, B, G, 1)
