@@ -103,3 +103,14 @@ def test_raw_entries_take_any_whole_number(cuda, number):
         assert torch.equal(ops.matmul_matgptq_grouped_raw(x, [words], [scales], np.array([N]), K, np.array([B], dtype=np.uint8), G, 1), want)
     with pytest.raises(RuntimeError):
         ops.matmul_matgptq_raw(x, words, scales, float(N), K, B, G, 1)
+
+
+@pytest.mark.gpu
+def test_pybind_stand_in_is_outside_autograd(cuda):
+    from matgptq_cuda import _CUDA
+    words, scales = _tensors(cuda)
+    grad = scales.clone().requires_grad_()
+    x = torch.ones(2, K, dtype=torch.float16, device=cuda, requires_grad=True)
+    assert not _CUDA.reorder_matgptq_scales(grad, N, K, G).requires_grad
+    y = _CUDA.matmul_matgptq(x, words, grad, N, K, B, G, 1)
+    assert not y.requires_grad and torch.equal(y, _matmul(x.detach(), words, scales))
