@@ -380,7 +380,9 @@ TORCH_LIBRARY_IMPL(matgptq_cuda, ADInplaceOrView, m) {
 // ---- Python module --------------------------------------------------------------------------------------------
 namespace {
 
-struct WithoutGil {  // a launch may wait for room in the stream's queue: other Python threads go on meanwhile
+// A launch may wait for room in the stream's queue, and an allocation for the device: other Python threads (and Python
+// callbacks that the stream is waiting for) go on meanwhile.
+struct WithoutGil {
   PyThreadState *state = PyEval_SaveThread();
   ~WithoutGil() { PyEval_RestoreThread(state); }
 };
@@ -437,17 +439,17 @@ PyObject *py_linear_forward(PyObject *, PyObject *const *args, Py_ssize_t nargs)
   int64_t rows = 1;
   for (size_t i = 0; i + 1 < sizes.size(); ++i) rows *= sizes[i];
   sizes.back() = v[0];
-  const bool as_is = input.is_contiguous() && reinterpret_cast<uintptr_t>(input.const_data_ptr()) % 16 == 0;
-  Tensor copy;
-  if (!as_is) {
-    const at::AutoDispatchBelowADInplaceOrView below;
-    copy = input.clone(at::MemoryFormat::Contiguous);
-  }
-  Tensor out = empty_on(sizes, type_of(v[4]), dev);
+  Tensor out;
   {
     const WithoutGil released;
+    Tensor copy;
+    if (!input.is_contiguous() || reinterpret_cast<uintptr_t>(input.const_data_ptr()) % 16 != 0) {
+      const at::AutoDispatchBelowADInplaceOrView below;
+      copy = input.clone(at::MemoryFormat::Contiguous);
+    }
+    out = empty_on(sizes, type_of(v[4]), dev);
     launch_matmul("matmul_matgptq", dev, v[2], v[3], v[0], v[1], rows, weights, scales,
-                  as_is ? input.const_data_ptr() : copy.const_data_ptr(), out.data_ptr(), v[4]);
+                  copy.defined() ? copy.const_data_ptr() : input.const_data_ptr(), out.data_ptr(), v[4]);
   }
   return THPVariable_Wrap(std::move(out));
   END_HANDLE_TH_ERRORS
@@ -498,9 +500,10 @@ PyObject *py_matmul_raw(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
   const c10::Device dev = x.device();
   const c10::cuda::CUDAGuard on_device(dev);
   const int64_t batch = x.size(-2);
-  Tensor out = args[8] == Py_None ? empty_on({batch, v[0]}, x.scalar_type(), dev) : THPVariable_Unpack(args[8]);
+  Tensor out = args[8] == Py_None ? Tensor() : THPVariable_Unpack(args[8]);
   {
     const WithoutGil released;
+    if (!out.defined()) out = empty_on({batch, v[0]}, x.scalar_type(), dev);
     launch_matmul("matgptq_b200_matmul", dev, v[2], v[3], v[0], v[1], batch, weights, scales, x.const_data_ptr(), out.data_ptr(), v[4]);
   }
   return THPVariable_Wrap(std::move(out));

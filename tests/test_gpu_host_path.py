@@ -1,5 +1,8 @@
 """MatGPTQLinear's C++ host path: the same rows as the operator computes, whatever form the input comes in, and the
 dispatcher still sees the call when something listens to it."""
+import ctypes
+import subprocess
+
 import pytest
 import torch
 from torch.utils._python_dispatch import TorchDispatchMode
@@ -106,3 +109,47 @@ def test_tensors_that_are_not_their_storage_take_the_operator(cuda, form):
     if form != "zero_tensor":  # it has no memory at all; the operator says what it thinks of that
         y = layer(x)
         assert torch.equal(torch.Tensor(y) if form == "subclass" else y, _op(layer, same))
+
+
+ALLOCATOR = """
+#include <cuda_runtime.h>
+extern "C" {
+int PyGILState_Check(void);
+int calls = 0, with_gil = 0;
+void *take(size_t size, int, cudaStream_t) {
+  ++calls;
+  with_gil += PyGILState_Check() != 0;
+  void *p = nullptr;
+  return cudaMalloc(&p, size) == cudaSuccess ? p : nullptr;
+}
+void give(void *p, size_t, int, cudaStream_t) { cudaFree(p); }
+}
+"""
+
+
+@pytest.mark.gpu
+def test_memory_is_allocated_without_the_gil(cuda, tmp_path):
+    # an allocation may wait for the device, and the device for a Python callback
+    from matgptq_b200 import ops
+    from matgptq_b200.build import _nvcc
+    (tmp_path / "allocator.cpp").write_text(ALLOCATOR)
+    path = str(tmp_path / "allocator.so")
+    subprocess.run([_nvcc(), "-shared", "-Xcompiler", "-fPIC", "-o", path, str(tmp_path / "allocator.cpp")], check=True)
+    counts = ctypes.CDLL(path)
+    calls, with_gil = ctypes.c_int.in_dll(counts, "calls"), ctypes.c_int.in_dll(counts, "with_gil")
+    allocator = torch.cuda.memory.CUDAPluggableAllocator(path, "take", "give")
+    layer = _layer(cuda)
+    args = (layer.matgptq_qweight, layer.matgptq_scales, layer.n_out_features, layer.n_in_features, layer.bitwidth, layer.group_size, 1)
+    base = torch.randn(12, 2 * layer.n_in_features, dtype=torch.float16, device=cuda)
+    x = base[:, :layer.n_in_features].contiguous()
+    for call in (lambda: layer(x), lambda: layer(base[:, :layer.n_in_features]), lambda: ops.matmul_matgptq_raw(x, *args),
+                 lambda: ops.matmul_matgptq_grouped_raw(x, *([a] for a in args[:3]), args[3], [args[4]], *args[5:]),
+                 lambda: torch.ops.matgptq_cuda.matmul_matgptq(x, *args)):
+        want, seen = call(), calls.value
+        pool = torch.cuda.MemPool(allocator.allocator())
+        with torch.cuda.use_mem_pool(pool):
+            y = call()
+        assert calls.value > seen and with_gil.value == 0
+        assert torch.equal(y, want)
+        torch.cuda.synchronize()
+        del y, pool
