@@ -4,7 +4,8 @@
 
 The library has no torch or Python dependency: it is the C-ABI boundary declared in
 ``include/matgptq_b200.h``.  Beside it the module ``_torch_ops.so`` (``csrc/torch_ops.cpp``) registers the torch
-operators on top of that ABI.  Objects are rebuilt only when a source or header is newer.
+operators on top of that ABI.  Objects are rebuilt only when a source or header is newer, the module also when torch,
+Python or its command line is another than it was built with.
 """
 from __future__ import annotations
 
@@ -21,6 +22,7 @@ LIB_PATH = os.path.join(PKG_DIR, "libmatgptq_b200.so")
 
 TORCH_OPS_SOURCE = os.path.join(CSRC, "torch_ops.cpp")
 TORCH_OPS_PATH = os.path.join(PKG_DIR, "_torch_ops.so")
+TORCH_OPS_STAMP = os.path.join(BUILD_DIR, "_torch_ops.txt")  # what the module was built with
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -65,6 +67,23 @@ def _torch_ops_command() -> list[str]:
             "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python"]
 
 
+def _torch_ops_built_with() -> str:
+    import torch
+    return "\n".join([torch.__version__, sys.version, *_torch_ops_command()])
+
+
+def _torch_ops_stale() -> bool:
+    """The module is bound to the ABI of the torch and Python that compiled it: an upgrade of either makes it stale
+    although no source is newer."""
+    if not os.path.exists(TORCH_OPS_PATH) or not os.path.exists(TORCH_OPS_STAMP):
+        return True
+    if os.path.getmtime(TORCH_OPS_PATH) < max(os.path.getmtime(TORCH_OPS_SOURCE),
+                                              os.path.getmtime(os.path.join(INCLUDE, "matgptq_b200.h"))):
+        return True
+    with open(TORCH_OPS_STAMP) as f:
+        return f.read() != _torch_ops_built_with()
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
     """Compile every ``.cu`` under ``csrc/`` and link the shared library, compile the operator module. Returns the
     library's path."""
@@ -85,11 +104,9 @@ def build(force: bool = False, verbose: bool = False) -> str:
                 cmd.insert(2, "-v")
                 print(" ".join(cmd), flush=True)
             procs.append((src, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)))
-    if (force or not os.path.exists(TORCH_OPS_PATH) or os.path.getmtime(TORCH_OPS_PATH) <
-            max(os.path.getmtime(TORCH_OPS_SOURCE), os.path.getmtime(os.path.join(INCLUDE, "matgptq_b200.h")))):
+    operators = None
+    if force or _torch_ops_stale():
         operators = subprocess.Popen(_torch_ops_command(), stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
-    else:
-        operators = None
     failed = False
     for src, proc in procs:
         out, _ = proc.communicate()
@@ -103,6 +120,9 @@ def build(force: bool = False, verbose: bool = False) -> str:
         if operators.returncode != 0:
             failed = True
             sys.stderr.write(f"--- g++ failed on torch_ops.cpp ---\n{out}\n")
+        else:
+            with open(TORCH_OPS_STAMP, "w") as f:
+                f.write(_torch_ops_built_with())
     if failed:
         raise RuntimeError("compilation failed")
     relink = force or procs or not os.path.exists(LIB_PATH)
