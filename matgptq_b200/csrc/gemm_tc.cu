@@ -26,6 +26,8 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <climits>
+
 #include "async.cuh"
 #include "decode.cuh"
 #include "host_util.h"
@@ -537,13 +539,64 @@ static int round_up16(int v) { return (v + 15) / 16 * 16; }
 constexpr int kTcHalfSmBytes = 112 * 1024;
 static bool tc_two_ctas_per_sm(int ncols) { return tc_plan(ncols, 3).total <= kTcHalfSmBytes; }
 
-// K split of the tensor-core path: one wave of CTAs over the SMs' slots; at least four blocks of K per CTA.
+// The batch goes in as few blocks of at most 256 rows as it takes, all of one size: a last block that is mostly empty
+// costs as much as a full one (300 rows as 2 x 160 instead of 256 + 44 in 256 columns: 8192 x 8192, 8 bits 71.0 -> 63.0 us).
+struct TcBatch {
+  int blocks;
+  int ncols;  // rows of a block rounded up to 16: UMMA N
+};
+static TcBatch tc_batch(int M) {
+  TcBatch b;
+  b.blocks = (M + 255) / 256;
+  b.ncols = round_up16((M + b.blocks - 1) / b.blocks);
+  return b;
+}
+
+// Clusters of `size` CTAs that run at once when each CTA has an SM to itself.  A cluster lies inside one GPC, so what is
+// left over in every GPC stays idle: fewer than SMs / size.  Asked once per device (two threads that race store the same
+// value); no limit where the device cannot tell.
+static int tc_clusters_at_once(int size) {
+  static std::atomic<int> cache[kMaxDevices][9];
+  static SharedMemoryOptIn opt_in;
+  const auto kernel = gemm_tc_kernel<4, 128, true, 16>;  // any instantiation: all of them fill an SM
+  int dev = 0;
+  if (size < 1 || size > 8 || current_device(&dev) != MG_OK) return INT_MAX;
+  int v = cache[dev][size].load(std::memory_order_relaxed);
+  if (v > 0) return v;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(1, static_cast<unsigned>(size), 1);
+  cfg.blockDim = dim3(18 * 32, 1, 1);
+  cfg.dynamicSmemBytes = 2 * kTcHalfSmBytes;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 1;
+  attr[0].val.clusterDim.y = static_cast<unsigned>(size);
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (opt_in.ensure(kernel, 2 * kTcHalfSmBytes) != MG_OK || cudaOccupancyMaxActiveClusters(&v, kernel, &cfg) != cudaSuccess) {
+    (void)cudaGetLastError();
+    v = 0;
+  }
+  if (v <= 0) v = INT_MAX;
+  cache[dev][size].store(v, std::memory_order_relaxed);
+  return v;
+}
+
+// K split of the tensor-core path: one wave of CTAs over the SMs' slots; at least four blocks of K per CTA.  Above 256 rows
+// the plan is for one CTA per SM.  Where the batch blocks are smaller than 256 rows, the wave has to hold as whole clusters
+// too: with blocks of one size a second wave takes as long as the first (with 256 + 1 rows it was the short block's).
+// N = 1024, K = 4096, 4 bits: 257 rows 16.5 us in 16 clusters of 8, 10.6 in clusters of 6; 520 rows 20.4 in 24 clusters of
+// 6, 12.9 in clusters of 5.  Full blocks of 256 rows keep the plan of one wave of CTAs, and so the order of their sums.
 int gemm_tc_pick_split(int N, int K, int M, int sm_count) {
-  const int ctas = ((N + 127) / 128) * ((M + 255) / 256);
+  const TcBatch batch = tc_batch(M);
+  const int ctas = ((N + 127) / 128) * batch.blocks;
   const int kblocks = K / 128;
-  const int want = tc_two_ctas_per_sm(round_up16(M < 256 ? M : 256)) ? 2 * sm_count : sm_count;
+  const int want = batch.blocks == 1 && tc_two_ctas_per_sm(batch.ncols) ? 2 * sm_count : sm_count;
   int split = 1;
   while (split < 8 && ctas * (split + 1) <= want && kblocks / (split + 1) >= 4) ++split;  // one wave
+  if (batch.blocks > 1 && batch.ncols < 256)
+    while (split > 1 && ctas > tc_clusters_at_once(split)) --split;
   return split;
 }
 
@@ -603,7 +656,7 @@ static int launch_gemm_tc_warps(GemmParams p, cudaStream_t stream, bool pdl, flo
     if (st != MG_OK) return st;
   }
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((p.N + 127) / 128, p.split, (p.M + 255) / 256);
+  cfg.gridDim = dim3((p.N + 127) / 128, p.split, tc_batch(p.M).blocks);
   cfg.blockDim = dim3((PW + 2) * 32, 1, 1);
   cfg.dynamicSmemBytes = plan.total;
   cfg.stream = stream;
@@ -657,16 +710,14 @@ static int launch_gemm_tc_warps(GemmParams p, cudaStream_t stream, bool pdl, flo
 // are no more CTAs than SMs.
 template <int B, int GS, bool BF16>
 static int launch_gemm_tc(GemmParams p, cudaStream_t stream, bool pdl, float *fallback_partial) {
-  // The batch goes in as few blocks of at most 256 rows as it takes, all of one size: a last block that is mostly empty
-  // costs as much as a full one (300 rows as 2 x 160 instead of 256 + 44 in 256 columns: 8192 x 8192, 8 bits 71.0 -> 63.0 us).
-  const int blocks = (p.M + 255) / 256;
-  p.ncols = round_up16((p.M + blocks - 1) / blocks);
+  const TcBatch batch = tc_batch(p.M);
+  p.ncols = batch.ncols;
   int sm_count = 0;
   {
     const int st = current_device_sm_count(&sm_count);
     if (st != MG_OK) return st;
   }
-  const long long ctas = static_cast<long long>((p.N + 127) / 128) * p.split * ((p.M + 255) / 256);
+  const long long ctas = static_cast<long long>((p.N + 127) / 128) * p.split * batch.blocks;
   if (!tc_two_ctas_per_sm(p.ncols) || ctas <= sm_count) return launch_gemm_tc_warps<B, GS, BF16, 16>(p, stream, pdl, fallback_partial);
   return launch_gemm_tc_warps<B, GS, BF16, 8>(p, stream, pdl, fallback_partial);
 }

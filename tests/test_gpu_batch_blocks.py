@@ -15,7 +15,10 @@ pytestmark = pytest.mark.gpu
     (8, -1, 2064, 640, 300),     # 2 x 160
     (3, 128, 1024, 4096, 512),   # full blocks, K split
     (6, 128, 4096, 1024, 513),   # three blocks of 176
-    (4, 128, 14336, 256, 1025)])
+    (4, 128, 14336, 256, 1025),
+    (4, 128, 1024, 4096, 257),   # K split limited by the clusters that run at once
+    (2, 32, 1040, 2048, 520),
+    (8, -1, 2048, 2048, 520)])
 def test_blocks_of_a_batch(cuda, dtype, b, gs, n_out, n_in, m):
     gen = torch.Generator(device=cuda).manual_seed(m)
     flag = 1 | (2 if dtype == torch.bfloat16 else 0)
@@ -30,3 +33,34 @@ def test_blocks_of_a_batch(cuda, dtype, b, gs, n_out, n_in, m):
     y = torch.ops.matgptq_cuda.matmul_matgptq(x, packed, s, n_out, n_in, b, gs, flag)
     assert _native.device_status() == 0
     assert torch.equal(y, (x.double() @ w.double().t()).to(dtype))
+
+
+def _replay_us(call, launches=16):
+    call()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        for _ in range(launches):
+            call()
+    best = float("inf")
+    for _ in range(8):
+        start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        start.record()
+        graph.replay()
+        end.record()
+        end.synchronize()
+        best = min(best, start.elapsed_time(end) * 1e3 / launches)
+    return best
+
+
+@pytest.mark.parametrize("m", [257, 520])
+def test_planned_split_runs_in_one_wave(cuda, m):
+    # 16 clusters of 8 CTAs fill 128 of 148 SMs, but not with whole clusters in every GPC: a second wave takes as long as the
+    # first (1.6 times the time of the split by 4 here)
+    n, k = 1024, 4096
+    words = torch.randint(-2 ** 31, 2 ** 31 - 1, (4 * n * k // 32,), device=cuda, dtype=torch.int32).view(torch.uint32)
+    scales = torch.full((n, k // 128), 2.0 ** -8, dtype=torch.bfloat16, device=cuda)
+    x = torch.randn(m, k, device=cuda).to(torch.bfloat16)
+    out = torch.empty(m, n, dtype=torch.bfloat16, device=cuda)
+    times = [_replay_us(lambda: ops.matmul_matgptq_raw(x, words, scales, n, k, 4, 128, 3, out=out, path=2, split_k=s)) for s in (0, 4)]
+    assert times[0] <= 1.3 * times[1], times
