@@ -181,32 +181,43 @@ template <int OFF> __device__ __forceinline__ void sts_v4(uint32_t addr, const u
                : "memory");
 }
 
+// Raw scales of rows g (lo) and g+8 (hi) for the groups of a block
+template <int GS> struct TcRaw {
+  uint16_t lo[TcScales<GS>::NG], hi[TcScales<GS>::NG];
+};
+
+// dense_scale() of both rows for one group
+struct TcGroup {
+  uint32_t lo, hi;
+};
+template <int B, int GS, bool BF16> __device__ __forceinline__ TcGroup tc_group(const TcRaw<GS> &r, int i) {
+  return TcGroup{dense_scale<B, BF16>(r.lo[i]), dense_scale<B, BF16>(r.hi[i])};
+}
+
 // Chunk JJ (0..3, 32 in-features) of a block: this lane's dense weights of rows g (lo) and g+8 (hi), eight each, as
 // 16 bytes per row into the A tile whose lane address for chunk 0 is `addr`.
 template <int B, bool BF16, int JJ>
-__device__ __forceinline__ void tc_store_chunk(const uint32_t (&w)[2 * B], uint32_t s_lo, uint32_t s_hi, uint32_t addr) {
+__device__ __forceinline__ void tc_store_chunk(const uint32_t (&w)[2 * B], const TcGroup &g, uint32_t addr) {
   uint4 lo, hi;
-  lo.x = dense_pair<B, BF16>(w, 8 * JJ + 0, s_lo);
-  lo.y = dense_pair<B, BF16>(w, 8 * JJ + 2, s_lo);
-  lo.z = dense_pair<B, BF16>(w, 8 * JJ + 4, s_lo);
-  lo.w = dense_pair<B, BF16>(w, 8 * JJ + 6, s_lo);
-  hi.x = dense_pair<B, BF16>(w, 8 * JJ + 1, s_hi);
-  hi.y = dense_pair<B, BF16>(w, 8 * JJ + 3, s_hi);
-  hi.z = dense_pair<B, BF16>(w, 8 * JJ + 5, s_hi);
-  hi.w = dense_pair<B, BF16>(w, 8 * JJ + 7, s_hi);
+  lo.x = dense_pair<B, BF16>(w, 8 * JJ + 0, g.lo);
+  lo.y = dense_pair<B, BF16>(w, 8 * JJ + 2, g.lo);
+  lo.z = dense_pair<B, BF16>(w, 8 * JJ + 4, g.lo);
+  lo.w = dense_pair<B, BF16>(w, 8 * JJ + 6, g.lo);
+  hi.x = dense_pair<B, BF16>(w, 8 * JJ + 1, g.hi);
+  hi.y = dense_pair<B, BF16>(w, 8 * JJ + 3, g.hi);
+  hi.z = dense_pair<B, BF16>(w, 8 * JJ + 5, g.hi);
+  hi.w = dense_pair<B, BF16>(w, 8 * JJ + 7, g.hi);
   sts_v4<(JJ & 1) * 4 * kTcChunkStride>(addr, lo);
   sts_v4<(JJ & 1) * 4 * kTcChunkStride + 128>(addr, hi);
 }
 
-// Half H (0, 1) of a block = chunks 2H and 2H+1 = one pipeline stage; slo/shi: raw scales of rows g and g+8
+// Half H (0, 1) of a block = chunks 2H and 2H+1 = one pipeline stage
 template <int B, int GS, bool BF16, int H>
-__device__ __forceinline__ void tc_store_half(const uint32_t (&w)[2 * B], const uint16_t (&slo)[TcScales<GS>::NG],
-                                              const uint16_t (&shi)[TcScales<GS>::NG], uint32_t addr) {
+__device__ __forceinline__ void tc_store_half(const uint32_t (&w)[2 * B], const TcRaw<GS> &raw, uint32_t addr) {
   constexpr int g0 = (GS == 32) ? 2 * H : 0, g1 = (GS == 32) ? 2 * H + 1 : 0;
-  const uint32_t lo0 = dense_scale<B, BF16>(slo[g0]), hi0 = dense_scale<B, BF16>(shi[g0]);
-  tc_store_chunk<B, BF16, 2 * H>(w, lo0, hi0, addr);
-  const uint32_t lo1 = (GS == 32) ? dense_scale<B, BF16>(slo[g1]) : lo0, hi1 = (GS == 32) ? dense_scale<B, BF16>(shi[g1]) : hi0;
-  tc_store_chunk<B, BF16, 2 * H + 1>(w, lo1, hi1, addr);
+  const TcGroup a = tc_group<B, GS, BF16>(raw, g0);
+  tc_store_chunk<B, BF16, 2 * H>(w, a, addr);
+  tc_store_chunk<B, BF16, 2 * H + 1>(w, (GS == 32) ? tc_group<B, GS, BF16>(raw, g1) : a, addr);
 }
 
 struct TcProducer {
@@ -219,11 +230,10 @@ struct TcProducer {
 // over, move on to the next stage.  `mine` false: the half belongs to the other warp of the pair.
 template <int B, int GS, bool BF16, int H>
 __device__ __forceinline__ bool tc_producer_half(TcProducer &pr, bool mine, bool valid, int lane, const uint32_t (&w)[2 * B],
-                                                 const uint16_t (&slo)[TcScales<GS>::NG],
-                                                 const uint16_t (&shi)[TcScales<GS>::NG]) {
+                                                 const TcRaw<GS> &raw) {
   if (mine) {
     if (!mbar_wait(pr.bar_empty + pr.idx8, pr.parity)) return false;  // the tensor pipe is done with what this stage held
-    if (valid) tc_store_half<B, GS, BF16, H>(w, slo, shi, pr.a_lane + pr.off);
+    if (valid) tc_store_half<B, GS, BF16, H>(w, raw, pr.a_lane + pr.off);
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic-proxy stores -> tensor pipe reads
     __syncwarp();
     if (lane == 0) mbar_arrive(pr.bar_full + pr.idx8);
@@ -305,24 +315,25 @@ __device__ __forceinline__ void gemm_tc_body(const GemmParams &p, const CUtensor
     // modulo by the (runtime) number of stages.
     constexpr int kAhead = (B >= 6) ? 3 : (PW == 16 ? 4 : 6);
     const uint32_t *wnext = p.w + (static_cast<size_t>(valid ? tile16 : 0) * p.kblocks + kb_lo) * BW;  // next block to load
-    const uint16_t *snext = p.s + (static_cast<size_t>(valid ? tile16 : 0) * groups + ((GS == -1) ? 0 : kb_lo * NG)) * 16 + g;
+    const size_t s_first = (static_cast<size_t>(valid ? tile16 : 0) * groups + ((GS == -1) ? 0 : kb_lo * NG)) * 16 + g;
+    const uint16_t *snext = p.s + s_first;
     uint32_t wq[kAhead][2 * B];
     // raw scales of rows g and g+8, loaded with the block's words and only touched when the block is decoded
     // (dense_scale() applied on arrival would stall the warp on the load it has just issued)
-    uint16_t sq_lo[kAhead][NG], sq_hi[kAhead][NG];
-    auto load_next = [&](uint32_t (&wdst)[2 * B], uint16_t (&lo)[NG], uint16_t (&hi)[NG]) {
+    TcRaw<GS> sq[kAhead];
+    auto load_next = [&](uint32_t (&wdst)[2 * B], TcRaw<GS> &raw) {
       load_block<B>(wnext, lane, wdst);
 #pragma unroll
       for (int j = 0; j < NG; ++j) {
-        lo[j] = ldg_u16_tc(snext + j * 16);
-        hi[j] = ldg_u16_tc(snext + j * 16 + 8);
+        raw.lo[j] = ldg_u16_tc(snext + j * 16);
+        raw.hi[j] = ldg_u16_tc(snext + j * 16 + 8);
       }
       wnext += BW;
       if (GS != -1) snext += NG * 16;
     };
 #pragma unroll
     for (int a = 0; a < kAhead; ++a)
-      if (valid && a < nblk) load_next(wq[a], sq_lo[a], sq_hi[a]);
+      if (valid && a < nblk) load_next(wq[a], sq[a]);
 
     // this lane's 16 bytes of rows g and g+8 in the A tile of stage 0, chunk t (shared-memory address)
     const uint32_t a_lane = base_u32 + plan.off_stages + plan.b_stage_bytes + t * kTcChunkStride + (2 * ptile) * 128 + g * 16;
@@ -340,11 +351,11 @@ __device__ __forceinline__ void gemm_tc_body(const GemmParams &p, const CUtensor
 #pragma unroll
       for (int a = 0; a < kAhead; ++a) {
         if (blk + a < nblk && !failed) {
-          if (!tc_producer_half<B, GS, BF16, 0>(pr, PW == 8 || my_half == 0, valid, lane, wq[a], sq_lo[a], sq_hi[a]) ||
-              !tc_producer_half<B, GS, BF16, 1>(pr, PW == 8 || my_half == 1, valid, lane, wq[a], sq_lo[a], sq_hi[a])) {
+          if (!tc_producer_half<B, GS, BF16, 0>(pr, PW == 8 || my_half == 0, valid, lane, wq[a], sq[a]) ||
+              !tc_producer_half<B, GS, BF16, 1>(pr, PW == 8 || my_half == 1, valid, lane, wq[a], sq[a])) {
             failed = true;
           } else if (valid && blk + a + kAhead < nblk) {
-            load_next(wq[a], sq_lo[a], sq_hi[a]);  // this block's registers are free: fetch the block kAhead ahead
+            load_next(wq[a], sq[a]);  // this block's registers are free: fetch the block kAhead ahead
           }
         }
       }
