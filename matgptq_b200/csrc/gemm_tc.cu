@@ -585,11 +585,10 @@ static int tc_clusters_at_once(int size) {
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  if (opt_in.ensure(kernel, 2 * kTcHalfSmBytes) != MG_OK || cudaOccupancyMaxActiveClusters(&v, kernel, &cfg) != cudaSuccess) {
+  if (opt_in.ensure(kernel, 2 * kTcHalfSmBytes) != MG_OK || cudaOccupancyMaxActiveClusters(&v, kernel, &cfg) != cudaSuccess || v <= 0) {
     (void)cudaGetLastError();
-    v = 0;
+    return INT_MAX;
   }
-  if (v <= 0) v = INT_MAX;
   cache[dev][size].store(v, std::memory_order_relaxed);
   return v;
 }

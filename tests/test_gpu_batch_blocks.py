@@ -1,5 +1,9 @@
 """Batches of several blocks on the tensor-core path, at the edges of the blocks: integer-valued weights and activations make
 every sum exact, so the product of the dense weights in fp64 is the expected result bit for bit."""
+import os
+import subprocess
+import sys
+
 import pytest
 import torch
 
@@ -64,3 +68,31 @@ def test_planned_split_runs_in_one_wave(cuda, m):
     out = torch.empty(m, n, dtype=torch.bfloat16, device=cuda)
     times = [_replay_us(lambda: ops.matmul_matgptq_raw(x, words, scales, n, k, 4, 128, 3, out=out, path=2, split_k=s)) for s in (0, 4)]
     assert times[0] <= 1.3 * times[1], times
+
+
+CAPTURED = """
+import torch
+from matgptq_b200 import _native, ops
+n, k, m = 1024, 4096, 300
+words = torch.randint(-2 ** 31, 2 ** 31 - 1, (3 * n * k // 32,), device="cuda", dtype=torch.int32).view(torch.uint32)
+scales = torch.full((n, k // 128), 2.0 ** -8, dtype=torch.float16, device="cuda")
+x = torch.randn(m, k, device="cuda").half()
+out, want = torch.empty(m, n, dtype=torch.float16, device="cuda"), torch.empty(m, n, dtype=torch.float16, device="cuda")
+WARM_UP
+torch.cuda.synchronize()
+graph = torch.cuda.CUDAGraph()
+with torch.cuda.graph(graph):
+    ops.matmul_matgptq_raw(x, words, scales, n, k, 3, 128, 1, out=out)
+graph.replay()
+ops.matmul_matgptq_raw(x, words, scales, n, k, 3, 128, 1, out=want)
+torch.cuda.synchronize()
+assert _native.device_status() == 0 and torch.equal(out, want)
+"""
+
+
+@pytest.mark.parametrize("warm_up", ["", "ops.matmul_matgptq_raw(x[:100], words, scales, n, k, 3, 128, 1)"])
+def test_first_call_above_256_rows_may_be_captured(cuda, warm_up):
+    # the question how many clusters run at once is asked while the stream is captured, for a kernel not used before
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    run = subprocess.run([sys.executable, "-c", CAPTURED.replace("WARM_UP", warm_up)], cwd=root, capture_output=True, text=True, timeout=300)
+    assert run.returncode == 0, run.stderr[-2000:]
