@@ -7,8 +7,8 @@
 // What bounds a call with few rows is not the GPU but the host: registered from Python the operator took 45 us a call
 // (argument parsing, two Python frames of torch.library, checks, a context manager, ctypes) in front of 4 to 12 us of
 // kernel.  Here a call is parsed once, checked, allocates its result and launches; linear_forward() also leaves out the
-// dispatcher when nothing that listens to it is active (no dispatch or function mode, no functorch level, no tensor
-// subclass), which is what an eager MatGPTQLinear needs.
+// dispatcher when nothing that listens to it is active (no dispatch or function mode, no functorch level) and the tensors
+// are ordinary CUDA tensors, which is what an eager MatGPTQLinear needs.
 #include <ATen/EmptyTensor.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <ATen/ops/empty_like.h>
