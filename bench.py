@@ -9,7 +9,7 @@ back to back from a CUDA graph; the loop order (M, shape, b) puts 20 other weigh
 more than L2) between two uses of the same weights.  `value` is algorithmic GB/s of the whole step
 (bytes a call must move: planes + scales + activations + output).  With N > 1 the same sweep runs
 tensor-parallel: k/v and gate/up split N, q/o and down split K and all-reduce their partial outputs.
-Rank 0 prints one JSON line.
+Rank 0 prints one JSON line on stdout; the per-cell tables go to stderr as another.
 """
 from __future__ import annotations
 
@@ -552,6 +552,10 @@ def ours_main(args) -> None:
         line["cpu_baseline"] = {"value": round(cpu["value"], 4), "unit": UNIT, "cores": cpu["cores"], "kind": "port",
                                 "sample": cpu["sample"], "dequant_ms_per_step": round(cpu["dequant_ms_per_step"], 2),
                                 "matmul_ms_per_step": round(cpu["matmul_ms_per_step"], 2)}
+    # the tables are most of 22 kB: a reader of the last few kB of stdout would lose the start of the line
+    tables = {k: extra.pop(k) for k in ("cells", "tensor_core_cells") if k in extra}
+    if tables:
+        print(json.dumps(tables), file=sys.stderr, flush=True)
     line.update(extra)
     print(json.dumps(line), flush=True)
     if world > 1:
