@@ -84,12 +84,15 @@ static int matmul_impl(int64_t bitwidth, int64_t group_size, int64_t n_out, int6
   const bool tensor_core = path == 2 || (path == 0 && uses_tensor_cores(n_out, batch));
   int r;
   if (z) {
-    // zero points: every batch size runs on the GEMV family (more than 16 rows in passes of 16), which applies scale and
-    // zero point in fp32; the tensor-core path has the implicit zero point only.  Dense tiles with zero points were 3.7
-    // times as fast at 128 rows, but round s * (code - zero) to 16 bits: 1.4 times the error against 64 bits (K = 4096,
-    // 4 bits: fp16 2.1e-4 -> 3.0e-4, bf16 1.7e-3 -> 2.4e-3), and in fp16 an infinity where that product passes 65504.
+    // Zero points: the GEMV up to 16 rows, then the tensor-core path that scales in fp32 (gemm_ts.cu), which like the GEMV
+    // rounds no weight to 16 bits.  16 rows are one pass of the GEMV; at 17 it reads and decodes the weights twice.
+    // 4096 x 4096, 4 bits, GEMV against tensor cores in us: 16 rows 8.2 / 11.4, 32 rows 16.2 / 12.3, 128 rows 58.1 / 21.9.
     if (path > 1) return MG_ERR_UNSUPPORTED;
-    r = mg::gemv_zp_launch(static_cast<int>(bitwidth), static_cast<int>(group_size), static_cast<int>(n_out),
+    if (path == 0 && batch > 16)
+      r = mg::gemm_ts_launch(static_cast<int>(bitwidth), static_cast<int>(group_size), static_cast<int>(n_out), static_cast<int>(n_in),
+                             static_cast<int>(batch), w, s, z, x, y, bf16, pdl, cs);
+    else
+      r = mg::gemv_zp_launch(static_cast<int>(bitwidth), static_cast<int>(group_size), static_cast<int>(n_out),
                            static_cast<int>(n_in), static_cast<int>(batch), w, s, z, x, y, bf16, pdl, warps_per_cta, split_k, cs);
   } else if (tensor_core) {
     r = mg::gemm_tc_launch(static_cast<int>(bitwidth), static_cast<int>(group_size), static_cast<int>(n_out),
@@ -322,10 +325,13 @@ int matgptq_b200_device_status(int *status_out, int reset) {
   int d = 0;
   r = mg::gemv_zp_device_status(&d, reset);
   if (r != MG_OK) return r;
+  int f = 0;
+  r = mg::gemm_ts_device_status(&f, reset);
+  if (r != MG_OK) return r;
   int e = 0;
   r = mg::selftest_device_status(&e, reset);
   if (r != MG_OK) return r;
-  if (status_out) *status_out = a ? a : (b ? b : (d ? d : e));
+  if (status_out) *status_out = a ? a : (b ? b : (d ? d : (f ? f : e)));
   return MG_OK;
 }
 

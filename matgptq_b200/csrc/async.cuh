@@ -94,6 +94,29 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
   return mbar_wait_slow(bar, parity);
 }
 
+// The same for waits that a chain of stages hangs on: no sleep between polls, each of which may suspend the warp until the
+// phase completes (the time is an upper limit in nanoseconds).
+static __device__ __noinline__ bool mbar_wait_suspended(uint32_t bar, uint32_t parity) {
+  for (uint32_t it = 0; it < (1u << 16); ++it) {
+    uint32_t ok;
+    asm volatile(
+        "{\n"
+        "  .reg .pred p;\n"
+        "  mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n"
+        "  selp.u32 %0, 1, 0, p;\n"
+        "}\n"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity), "r"(20000u)
+        : "memory");
+    if (ok) return true;
+  }
+  return false;
+}
+__device__ __forceinline__ bool mbar_wait_chain(uint32_t bar, uint32_t parity) {
+  if (mbar_try_wait(bar, parity)) return true;
+  return mbar_wait_suspended(bar, parity);
+}
+
 __device__ __forceinline__ void report_status(int code) { atomicCAS(&g_device_status, 0, code); }
 
 }  // namespace mg

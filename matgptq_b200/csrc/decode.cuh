@@ -272,25 +272,33 @@ template <int B> __device__ __forceinline__ uint32_t dense_int_bf16(const uint32
   }
 }
 
+// Pair P of a lane as exact integers (code - Z) * DensePre<B> in the activations' type
+template <int B, bool BF16> __device__ __forceinline__ uint32_t dense_int(const uint32_t (&w)[2 * B], int P) {
+  if constexpr (BF16) {
+    return dense_int_bf16<B>(w, P);
+  } else {
+    const uint32_t x = field_pair<B>(w, P, kMagic);
+    switch (kstep_offset<B>(P >> 2)) {  // a compile-time constant once the caller's loops are unrolled
+      case 0: return dense_int_at<B, 0>(x);
+      case 2: return dense_int_at<B, 2>(x);
+      case 3: return dense_int_at<B, 3>(x);
+      case 4: return dense_int_at<B, 4>(x);
+      case 6: return dense_int_at<B, 6>(x);
+      default: return dense_int_at<B, 8>(x);
+    }
+  }
+}
+
 // scale2: dense_scale() of the row's scale
 template <int B, bool BF16>
 __device__ __forceinline__ uint32_t dense_pair(const uint32_t (&w)[2 * B], int P, uint32_t scale2) {
+  const uint32_t v = dense_int<B, BF16>(w, P);
   if constexpr (BF16) {
-    const uint32_t vb = dense_int_bf16<B>(w, P);
-    const __nv_bfloat162 r = __hmul2(*reinterpret_cast<const __nv_bfloat162 *>(&scale2), *reinterpret_cast<const __nv_bfloat162 *>(&vb));
+    const __nv_bfloat162 r = __hmul2(*reinterpret_cast<const __nv_bfloat162 *>(&scale2), *reinterpret_cast<const __nv_bfloat162 *>(&v));
     return *reinterpret_cast<const uint32_t *>(&r);
+  } else {
+    return h2_bits(__hmul2(bits_h2(scale2), bits_h2(v)));
   }
-  const uint32_t x = field_pair<B>(w, P, kMagic);
-  uint32_t v;
-  switch (kstep_offset<B>(P >> 2)) {  // a compile-time constant once the caller's loops are unrolled
-    case 0: v = dense_int_at<B, 0>(x); break;
-    case 2: v = dense_int_at<B, 2>(x); break;
-    case 3: v = dense_int_at<B, 3>(x); break;
-    case 4: v = dense_int_at<B, 4>(x); break;
-    case 6: v = dense_int_at<B, 6>(x); break;
-    default: v = dense_int_at<B, 8>(x); break;
-  }
-  return h2_bits(__hmul2(bits_h2(scale2), bits_h2(v)));
 }
 
 // Coalesced load of a lane's words of one block (all lanes of a warp call it).

@@ -32,6 +32,7 @@
 #include "decode.cuh"
 #include "host_util.h"
 #include "kernels.h"
+#include "tc_common.cuh"
 
 namespace mg {
 
@@ -54,94 +55,6 @@ struct GemmParams {
   int stages;
 };
 
-// TMA load of one box of a 2-D tensor map into shared memory; x (the innermost coordinate) times the element
-// size must be a multiple of 16 bytes: here x is a multiple of 64 two-byte elements.
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, int x, int y, uint32_t bar) {
-  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
-               "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(bar)
-               : "memory");
-}
-
-// 64-bit shared-memory matrix descriptor (K-major).  layout_type: 0 = no swizzle, 2 = 128-byte swizzle.
-__device__ __forceinline__ uint64_t umma_smem_desc(uint32_t addr, uint32_t lbo_bytes, uint32_t sbo_bytes, uint32_t layout_type) {
-  uint64_t d = 0;
-  d |= static_cast<uint64_t>((addr >> 4) & 0x3FFFu);
-  d |= static_cast<uint64_t>((lbo_bytes >> 4) & 0x3FFFu) << 16;
-  d |= static_cast<uint64_t>((sbo_bytes >> 4) & 0x3FFFu) << 32;
-  d |= 1ull << 46;  // descriptor version of this architecture
-  d |= static_cast<uint64_t>(layout_type & 7u) << 61;
-  return d;
-}
-
-// 32-bit instruction descriptor: fp32 accumulate, A and B both K-major, both fp16 (0) or bf16 (1).
-__host__ __device__ inline uint32_t umma_instr_desc(int fmt, int n) {
-  return (1u << 4) | (static_cast<uint32_t>(fmt) << 7) | (static_cast<uint32_t>(fmt) << 10) |
-         (static_cast<uint32_t>(n >> 3) << 17) | (static_cast<uint32_t>(128 >> 4) << 24);
-}
-
-__device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n"
-      "  .reg .pred p;\n"
-      "  setp.ne.b32 p, %4, 0;\n"
-      "  tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
-      "}\n" ::"r"(tmem_d),
-      "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
-// true in exactly one lane of a converged warp
-__device__ __forceinline__ bool elect_one() {
-  uint32_t pred;
-  asm volatile(
-      "{\n"
-      "  .reg .pred p;\n"
-      "  elect.sync _|p, 0xffffffff;\n"
-      "  selp.u32 %0, 1, 0, p;\n"
-      "}\n"
-      : "=r"(pred));
-  return pred != 0;
-}
-
-__device__ __forceinline__ void umma_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-        "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]),
-        "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]),
-        "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-      : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-
-template <bool BF16> __device__ __forceinline__ uint16_t to_out16(float f) {
-  return BF16 ? __bfloat16_as_ushort(__float2bfloat16_rn(f)) : __half_as_ushort(__float2half_rn(f));
-}
-
-// every thread of every CTA of the cluster; orders shared-memory writes before the other CTAs' reads
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
-// address of this CTA's shared-memory location `addr` in the CTA of rank `cta` of the cluster
-__device__ __forceinline__ uint32_t map_to_cta(uint32_t addr, int cta) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(cta));
-  return r;
-}
-
-__device__ __forceinline__ float4 ld_cluster_f32x4(uint32_t addr) {
-  float4 v;
-  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
-  return v;
-}
-
 // shared-memory plan (host and device)
 struct TcPlan {
   int b_stage_bytes, stage_bytes, off_stages, total;
@@ -153,21 +66,6 @@ __host__ __device__ inline TcPlan tc_plan(int ncols, int stages) {
   p.off_stages = 1024;                                         // barriers and the TMEM address live below
   p.total = p.off_stages + stages * p.stage_bytes + 1024;      // slack to align the dynamic base to 1024
   return p;
-}
-
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-        "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-      : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-
-__device__ __forceinline__ uint16_t ldg_u16_tc(const uint16_t *p) {
-  uint16_t r;
-  asm volatile("ld.global.nc.u16 %0, [%1];" : "=h"(r) : "l"(p));
-  return r;
 }
 
 // scale groups per 128-wide block
@@ -566,7 +464,7 @@ static TcBatch tc_batch(int M) {
 // Clusters of `size` CTAs that run at once when each CTA has an SM to itself.  A cluster lies inside one GPC, so what is
 // left over in every GPC stays idle: fewer than SMs / size.  Asked once per device (two threads that race store the same
 // value); no limit where the device cannot tell.
-static int tc_clusters_at_once(int size) {
+int tc_clusters_at_once(int size) {
   static std::atomic<int> cache[kMaxDevices][9];
   static SharedMemoryOptIn opt_in;
   const auto kernel = gemm_tc_kernel<4, 128, true, 16>;  // any instantiation: all of them fill an SM
@@ -617,8 +515,8 @@ long long gemm_tc_workspace_bytes(int N, int K, int M, int sm_count) {
 }
 
 // Tensor map of the activations x[M, K] (two-byte elements, row-major) with boxes of 64 in-features x `box_rows`
-// batch rows and the 128-byte swizzle the UMMA descriptor of the B operand expects; rows past M read as zeros.
-static int make_x_tensor_map(CUtensorMap *map, const void *x, int M, int K, int box_rows) {
+// batch rows and, where the UMMA descriptor of the B operand expects it, the 128-byte swizzle; rows past M read as zeros.
+int tc_make_x_tensor_map(CUtensorMap *map, const void *x, int M, int K, int box_rows, bool swizzled) {
   typedef CUresult (*EncodeTiled)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
                                   const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -635,7 +533,8 @@ static int make_x_tensor_map(CUtensorMap *map, const void *x, int M, int K, int 
   const cuuint32_t box[2] = {64u, static_cast<cuuint32_t>(box_rows)};
   const cuuint32_t estride[2] = {1u, 1u};
   const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, const_cast<void *>(x), gdim, gstride, box, estride,
-                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                            CU_TENSOR_MAP_INTERLEAVE_NONE,
+                            swizzled ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? MG_OK : MG_ERR_CUDA;
 }
@@ -656,7 +555,7 @@ template <int B, int GS, bool BF16, int PW>
 static int launch_gemm_tc_warps(GemmParams p, cudaStream_t stream, bool pdl, float *fallback_partial) {
   auto kernel = gemm_tc_kernel<B, GS, BF16, PW>;
   CUtensorMap xmap;
-  if (make_x_tensor_map(&xmap, p.x, p.M, p.K, p.ncols) != MG_OK) return MG_ERR_CUDA;
+  if (tc_make_x_tensor_map(&xmap, p.x, p.M, p.K, p.ncols, true) != MG_OK) return MG_ERR_CUDA;
   const int stages = tc_pick_stages(p.ncols, PW);
   p.stages = stages;
   const TcPlan plan = tc_plan(p.ncols, stages);

@@ -63,6 +63,14 @@ int gemm_tc_launch(int bitwidth, int group_size, int N, int K, int M, const void
                    void *y, void *workspace, long long workspace_bytes, bool bf16, bool pdl, int split_override,
                    cudaStream_t stream, int ldy = 0, bool scratch_reduce = false);
 int gemm_tc_device_status(int *status_out, int reset);
+// Clusters of `size` CTAs (1 to 8) that run at once on the current device when each CTA has an SM to itself; INT_MAX where
+// the device cannot tell.
+int tc_clusters_at_once(int size);
+
+// gemm_ts.cu
+int gemm_ts_launch(int bitwidth, int group_size, int N, int K, int M, const void *w, const void *s, const void *z, const void *x,
+                   void *y, bool bf16, bool pdl, cudaStream_t stream, int ldy = 0);
+int gemm_ts_device_status(int *status_out, int reset);
 
 // selftest.cu
 int selftest_device_status(int *status_out, int reset);

@@ -1,0 +1,40 @@
+"""Tensor-core path with the weights in tensor memory and fp32 scaling: edges of its row tiles, batch blocks, stages and K
+splits, against the unrounded weights in 64 bits."""
+import pytest
+import torch
+
+from matgptq_b200 import _native, ops, synth  # noqa: F401  registers the operators
+from oracle import matgptq_oracle as oracle
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("b,gs,n_out,n_in,m", [
+    (2, 128, 16, 128, 17),       # one tile, one block of in-features
+    (3, 32, 144, 384, 33),       # a last CTA with one tile of its eight
+    (4, 128, 1040, 2944, 32),    # sixteen or eight tiles a CTA, K split unevenly
+    (6, -1, 2064, 1152, 48),
+    (8, 32, 272, 640, 64),
+    (4, 128, 4096, 4096, 65),    # two batch blocks of 48 rows
+    (8, -1, 256, 4224, 129),     # three blocks
+    (2, 128, 28672, 256, 20),    # more tiles than one wave of eight a CTA holds
+    (3, 128, 1024, 14336, 128)])
+def test_zero_points_at_the_edges(cuda, dtype, b, gs, n_out, n_in, m):
+    flag = 1 | (2 if dtype == torch.bfloat16 else 0)
+    layer = synth.make_layer(n_out, n_in, gs, seed=b, sym=False, dtype=dtype, device=cuda)
+    x = synth.make_activations(m, n_in, seed=m, dtype=dtype, device=cuda)
+    packed = torch.ops.matgptq_cuda.slice_pack_matgptq_qweights(layer.qweight, n_out, n_in, 8, b, gs, flag)
+    s, z = (torch.ops.matgptq_cuda.reorder_matgptq_scales(t, n_out, n_in, gs) for t in (layer.scales, layer.zeros))
+    y = torch.ops.matgptq_cuda.matmul_matgptq_zeros(x, packed, s, z, n_out, n_in, b, gs, flag)
+    again = torch.ops.matgptq_cuda.matmul_matgptq_zeros(x, packed, s, z, n_out, n_in, b, gs, flag)
+    assert _native.device_status() == 0
+    assert torch.equal(y, again)  # sums in a fixed order
+    codes = oracle.matryoshka_slice(layer.qweight, 8, b).double() * 2 ** (8 - b) - 128
+    group = n_in if gs == -1 else gs
+    scale, zero = (t.double().repeat_interleave(group, 1) for t in (layer.scales, layer.zeros))
+    ref = x.double() @ (scale * (codes - (zero - 128))).t()
+    # the result is rounded once; sums of the integers and of the activations meet in fp32, a few dozen additions of 2^-24 each
+    size = x.double().abs() @ (scale.abs() * (codes.abs() + (zero - 128).abs())).t()
+    half_ulp = 2.0 ** (-8 if dtype == torch.bfloat16 else -11)  # of a value just above a power of two: 7 and 10 bits follow it
+    assert ((y.double() - ref).abs() <= half_ulp * ref.abs() * 1.01 + 2.0 ** -19 * size).all()
