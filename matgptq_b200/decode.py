@@ -158,7 +158,6 @@ class PackedLlama:
         self.cos, self.sin = ang.cos(), ang.sin()
         self.k_cache = [torch.zeros(batch, self.kv_loc, max_seq, d, dtype=dtype, device=self.dev) for _ in range(shape.n_layers)]
         self.v_cache = [torch.zeros_like(k) for k in self.k_cache]
-        self.key_index = torch.arange(max_seq, device=self.dev)
 
     # -- pieces ------------------------------------------------------------------------------
     def linear(self, layer: int, which: str, x: torch.Tensor) -> torch.Tensor:
@@ -201,8 +200,8 @@ class PackedLlama:
         h = torch.empty_like(x)
         q = torch.empty(B, self.h_loc, S, d, dtype=self.dtype, device=self.dev)
         act = torch.empty(rows, self.layers[0]["down"].n_in, dtype=self.dtype, device=self.dev)
-        visible = self.key_index[None, :] <= positions[:, None]
-        mask = torch.zeros(S, self.max_seq, dtype=self.dtype, device=self.dev).masked_fill_(~visible, float("-inf"))[None, None]
+        mask = torch.empty(1, 1, S, self.max_seq, dtype=self.dtype, device=self.dev)
+        _native.check(lib.matgptq_b200_causal_mask(positions.data_ptr(), mask.data_ptr(), S, self.max_seq, flag, stream), "causal_mask")
         add_norm(x, None, self.layers[0]["ln1"], h)
         for li, L in enumerate(self.layers):
             qkv = self.linear(li, "qkv", h)

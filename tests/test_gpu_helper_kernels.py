@@ -36,6 +36,19 @@ def test_silu_mul(lib, cuda, dtype, rows, inter, shift):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("seq,keys", [(1, 256), (1, 1), (3, 13), (5, 1032), (5000, 16)])
+def test_causal_mask(lib, cuda, dtype, seq, keys):
+    pos = torch.randint(-1, keys + 2, (seq,), generator=torch.Generator(device=cuda).manual_seed(seq), device=cuda)
+    mask = torch.full((seq + 1, keys), 7.0, dtype=dtype, device=cuda)
+    flag = FLAG_BF16 if dtype == torch.bfloat16 else 0
+    assert lib.matgptq_b200_causal_mask(pos.data_ptr(), mask.data_ptr(), seq, keys, flag, torch.cuda.current_stream().cuda_stream) == 0
+    hidden = torch.arange(keys, device=cuda) > pos[:, None]
+    assert torch.equal(mask[:seq], torch.zeros(seq, keys, dtype=dtype, device=cuda).masked_fill_(hidden, float("-inf")))
+    assert (mask[seq] == 7.0).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("batch,seq,heads,kv,d,shift",
                          [(1, 1, 32, 8, 128, 0), (3, 5, 4, 2, 64, 0), (2, 7, 3, 1, 24, 0), (2, 3, 4, 2, 12, 0), (2, 3, 4, 2, 64, 1)])
 def test_rope_kv(lib, cuda, dtype, batch, seq, heads, kv, d, shift):
