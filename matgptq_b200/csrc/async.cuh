@@ -94,10 +94,14 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
   return mbar_wait_slow(bar, parity);
 }
 
-// The same for waits that a chain of stages hangs on: no sleep between polls, each of which may suspend the warp until the
-// phase completes (the time is an upper limit in nanoseconds).
-static __device__ __noinline__ bool mbar_wait_suspended(uint32_t bar, uint32_t parity) {
-  for (uint32_t it = 0; it < (1u << 16); ++it) {
+// The same for waits that a chain of stages hangs on, called by all lanes of a converged warp: no sleep between polls, each of
+// which may suspend the warp until the phase completes (the time is an upper limit in nanoseconds).  The lanes vote on every
+// poll, so that all of them leave together with one answer: what follows are warp-wide instructions (tcgen05.st and .ld,
+// mma.sync, elect.sync), and a flag that differed between lanes would send some of them past these.
+constexpr uint32_t kChainPolls = 1u << 16;
+
+static __device__ __noinline__ bool mbar_wait_suspended(uint32_t bar, uint32_t parity, uint32_t polls) {
+  for (uint32_t it = 0; it < polls; ++it) {
     uint32_t ok;
     asm volatile(
         "{\n"
@@ -108,13 +112,13 @@ static __device__ __noinline__ bool mbar_wait_suspended(uint32_t bar, uint32_t p
         : "=r"(ok)
         : "r"(bar), "r"(parity), "r"(20000u)
         : "memory");
-    if (ok) return true;
+    if (__all_sync(0xffffffffu, ok != 0)) return true;
   }
   return false;
 }
-__device__ __forceinline__ bool mbar_wait_chain(uint32_t bar, uint32_t parity) {
-  if (mbar_try_wait(bar, parity)) return true;
-  return mbar_wait_suspended(bar, parity);
+__device__ __forceinline__ bool mbar_wait_chain(uint32_t bar, uint32_t parity, uint32_t polls = kChainPolls) {
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  return mbar_wait_suspended(bar, parity, polls);
 }
 
 __device__ __forceinline__ void report_status(int code) { atomicCAS(&g_device_status, 0, code); }

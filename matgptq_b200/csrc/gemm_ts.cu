@@ -322,6 +322,7 @@ __global__ void __launch_bounds__(kTsWarps * 32, 1) gemm_ts_kernel(const TsParam
       }
       if (GS != -1 && blk + 1 < nblk) load_scales();
       const float *my_sums = sums + (GS == -1 ? 0 : sum_buf * 4 * kTsMaxCols);
+      __syncwarp();
       asm volatile("bar.sync 1, %0;" ::"n"(kTsScalers * 32) : "memory");  // the sums of block blk are there
       sum_buf = sum_buf == 2 ? 0 : sum_buf + 1;
       if (blk + 1 < nblk) sum_block(GS == -1 ? 0 : sum_buf, GS != -1 || blk + 2 == nblk);
@@ -359,6 +360,7 @@ __global__ void __launch_bounds__(kTsWarps * 32, 1) gemm_ts_kernel(const TsParam
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
         if (lane == 0) mbar_arrive(base + kTsBarDEmpty + 8 * buf);
+        if constexpr (NG > 1) __syncwarp();  // before the next group's reads
         d_ring.advance(1, accs);
       }
     }
@@ -477,9 +479,9 @@ __global__ void __launch_bounds__(kTsWarps * 32, 1) gemm_ts_kernel(const TsParam
   }
 
   // ---------------------------------------------------------------------- sums of a split K
+  __syncwarp();
   if (p.split > 1) {
     // The CTAs of one cluster share the tiles along K.  Each adds, in the order of the K ranges, the batch rows it owns.
-    __syncwarp();
     cluster_sync_all();
     if (warp < kFirstStager) {
       asm volatile("griddepcontrol.wait;" ::: "memory");

@@ -1,7 +1,8 @@
 // Self-test of the bounded waits: a wait that nothing will ever satisfy has to give up, record its status
 // code and let the kernel finish, so that the context stays usable.  The kernels of this library wait on
 // mbarriers that asynchronous copies complete (async.cuh); here one warp arms such a barrier for bytes that
-// no copy delivers and waits on it with a short poll limit.  Nothing is faulted, trapped or left spinning.
+// no copy delivers and waits on it with a short poll limit, in each of the ways that the kernels wait.  Nothing is
+// faulted, trapped or left spinning.
 // The reference has no counterpart (its only error path is exit(1), csrc/include/common.cuh:44-51).
 #include <cuda_runtime.h>
 
@@ -11,25 +12,34 @@
 
 namespace mg {
 
-__global__ void __launch_bounds__(32, 1) wait_timeout_probe_kernel(int code, unsigned polls, int *gave_up) {
-  __shared__ __align__(8) unsigned long long bar_storage;
-  const uint32_t bar = smem_u32(&bar_storage);
+// The warp waits with mbar_wait_bounded, then with mbar_wait_chain, where the odd lanes ask for a barrier whose phase is
+// complete: a warp has one answer there, so these give up as well.  *gave_up is set when every lane gave up both times.
+__global__ void __launch_bounds__(32, 1) wait_timeout_probe_kernel(int code, unsigned polls, unsigned chain_polls, int *gave_up) {
+  __shared__ __align__(8) unsigned long long bar_storage[2];
+  const uint32_t open = smem_u32(&bar_storage[0]), complete = smem_u32(&bar_storage[1]);
   if (threadIdx.x == 0) {
-    mbar_init(bar, 1);
+    mbar_init(open, 1);
+    mbar_init(complete, 1);
     mbar_init_fence();
   }
   __syncwarp();
-  if (threadIdx.x == 0) mbar_arrive_expect_tx(bar, 64);  // 64 bytes are expected; no copy is issued
+  if (threadIdx.x == 0) {
+    mbar_arrive_expect_tx(open, 64);  // 64 bytes are expected; no copy is issued
+    mbar_arrive(complete);
+  }
   __syncwarp();
-  const bool ok = mbar_wait_bounded(bar, 0, polls);
-  if (!ok) {
+  const bool bounded = mbar_wait_bounded(open, 0, polls);
+  __syncwarp();
+  const bool chain = mbar_wait_chain((threadIdx.x & 1) ? complete : open, 0, chain_polls);
+  __syncwarp();
+  if (__all_sync(0xffffffffu, !bounded && !chain)) {
     report_status(code);
     if (threadIdx.x == 0 && gave_up) *gave_up = 1;
   }
 }
 
-int selftest_wait_timeout_launch(int code, unsigned polls, int *gave_up, cudaStream_t stream) {
-  wait_timeout_probe_kernel<<<1, 32, 0, stream>>>(code, polls, gave_up);
+int selftest_wait_timeout_launch(int code, unsigned polls, unsigned chain_polls, int *gave_up, cudaStream_t stream) {
+  wait_timeout_probe_kernel<<<1, 32, 0, stream>>>(code, polls, chain_polls, gave_up);
   return cudaGetLastError() == cudaSuccess ? MG_OK : MG_ERR_CUDA;
 }
 
@@ -41,6 +51,6 @@ extern "C" int matgptq_b200_selftest_wait_timeout(int status_code, int *gave_up_
   if (status_code != mg::kStatusWeightCopyTimeout && status_code != mg::kStatusActivationCopyTimeout &&
       status_code != mg::kStatusMmaTimeout)
     return MG_ERR_BAD_ARG;
-  // 4096 polls of about 40 ns each and the hardware's own try_wait time-out: well under a second
-  return mg::selftest_wait_timeout_launch(status_code, 4096u, gave_up_flag, static_cast<cudaStream_t>(stream));
+  // 4096 polls of about 40 ns each and the hardware's own try_wait time-out, then 256 polls of at most 20 us: well under a second
+  return mg::selftest_wait_timeout_launch(status_code, 4096u, 256u, gave_up_flag, static_cast<cudaStream_t>(stream));
 }
