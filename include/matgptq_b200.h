@@ -274,6 +274,13 @@ int matgptq_b200_device_status(int *status_out, int reset);
  */
 int matgptq_b200_selftest_wait_timeout(int status_code, int *gave_up_flag, void *stream);
 
+/*
+ * Self-test of launch chains: a kernel that lets the kernel behind it start at once, rests for `rest_ms`
+ * milliseconds (at most 4000) and only then copies n 16-bit values from src to dst.  A product launched with
+ * FLAG_PDL right behind it has to wait for dst, however long that takes.  No counterpart in the reference.
+ */
+int matgptq_b200_selftest_late_writer(const void *src, void *dst, int64_t n, int rest_ms, void *stream);
+
 #ifdef __cplusplus
 }
 #endif

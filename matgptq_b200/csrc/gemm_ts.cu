@@ -201,7 +201,8 @@ __global__ void __launch_bounds__(kTsWarps * 32, 1) gemm_ts_kernel(const TsParam
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *reinterpret_cast<volatile uint32_t *>(base_ptr + kTsTmemSlot);
   // Weights, scales and zero points are never written by a kernel: only the activations and the results have to wait for
-  // the kernel before this one.
+  // the kernel before this one.  Every warp waits for it before its first wait on a barrier that hangs on the activations: that
+  // kernel may take longer than the limit of such a wait.
   asm volatile("griddepcontrol.launch_dependents;");
 
   // With K split the B stages hold [batch row][128 x row blocks out-feature slots] of sums once the last group is complete
@@ -213,11 +214,16 @@ __global__ void __launch_bounds__(kTsWarps * 32, 1) gemm_ts_kernel(const TsParam
     // ------------------------------------------------------------------ producers
     TsRing ring(0, 1);
     ring.advance(phase, stages);
+    bool ahead = true;  // in the first pass through the stages, which are free from the start
     const uint32_t a_lane = tmem + a_col0 + (static_cast<uint32_t>(quad * 32 + (j & 1) * 16) << 16) + (j >> 1) * 64;
     for (int kb = phase; kb < my_blocks; kb += step * kAhead) {
 #pragma unroll
       for (int a = 0; a < kAhead; ++a) {
         if (kb + a * step < my_blocks) {
+          if (ahead && ring.parity == 0) {
+            asm volatile("griddepcontrol.wait;" ::: "memory");
+            ahead = false;
+          }
           if (!failed && !mbar_wait_chain(base + kTsBarDone + 8 * ring.idx, ring.parity)) failed = true;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           const uint32_t taddr = a_lane + ring.idx * (rbs * 64);
@@ -267,6 +273,7 @@ __global__ void __launch_bounds__(kTsWarps * 32, 1) gemm_ts_kernel(const TsParam
       }
     };
     load_scales();
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // for the activations, and before anything is written
     TsRing b_ring(0, 0);
     const int sw = warp - kFirstScaler;
     float csum[NG][4];  // the groups' sums of the activations of batch rows 8 sw .. + 7
@@ -365,7 +372,6 @@ __global__ void __launch_bounds__(kTsWarps * 32, 1) gemm_ts_kernel(const TsParam
       }
     }
     if (failed) report_status(kStatusMmaTimeout);
-    asm volatile("griddepcontrol.wait;" ::: "memory");  // nothing is written before the previous kernel is done
     constexpr float kRest = static_cast<float>(1 << (8 - B)) / static_cast<float>(DensePre<B>::value);
     const int n = (tile0 + my_tile) * 16 + (lane & 15);
 #pragma unroll
@@ -395,6 +401,7 @@ __global__ void __launch_bounds__(kTsWarps * 32, 1) gemm_ts_kernel(const TsParam
     const uint32_t tile0_addr = base + kTsOffStages + h * b_half_bytes + sub * 128 + (ci & 1) * 8;
     const uint32_t c_even = ((((ci & 4) | ((ci >> 1) & 1)) ^ sub) << 4), c_odd = c_even ^ 64;  // rows sub and sub + 4 of eight
     TsRing ring(0, 1);
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     for (int blk = 0; blk < nblk; ++blk) {
       const int slot = blk & (kTsRawStages - 1);
       if (!failed && !mbar_wait_chain(base + kTsBarRawFull + 8 * slot, (blk / kTsRawStages) & 1)) failed = true;
@@ -484,7 +491,7 @@ __global__ void __launch_bounds__(kTsWarps * 32, 1) gemm_ts_kernel(const TsParam
     // The CTAs of one cluster share the tiles along K.  Each adds, in the order of the K ranges, the batch rows it owns.
     cluster_sync_all();
     if (warp < kFirstStager) {
-      asm volatile("griddepcontrol.wait;" ::: "memory");
+      asm volatile("griddepcontrol.wait;" ::: "memory");  // a producer with few blocks has not waited yet
       const int per = (p.ncols + p.split - 1) / p.split;
       const int c_lo = sk * per, c_hi = min(min(c_lo + per, p.ncols), mrows);
       const int vecs = slots / 4;  // four out-features a step

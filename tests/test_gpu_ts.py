@@ -38,3 +38,48 @@ def test_zero_points_at_the_edges(cuda, dtype, b, gs, n_out, n_in, m):
     size = x.double().abs() @ (scale.abs() * (codes.abs() + (zero - 128).abs())).t()
     half_ulp = 2.0 ** (-8 if dtype == torch.bfloat16 else -11)  # of a value just above a power of two: 7 and 10 bits follow it
     assert ((y.double() - ref).abs() <= half_ulp * ref.abs() * 1.01 + 2.0 ** -19 * size).all()
+
+
+def _zp_layer(n_out, n_in, b, gs, dtype, cuda):
+    layer = synth.make_layer(n_out, n_in, gs, seed=b, sym=False, dtype=dtype, device=cuda)
+    flag = 1 | (2 if dtype == torch.bfloat16 else 0)
+    packed = torch.ops.matgptq_cuda.slice_pack_matgptq_qweights(layer.qweight, n_out, n_in, 8, b, gs, flag)
+    s, z = (torch.ops.matgptq_cuda.reorder_matgptq_scales(t, n_out, n_in, gs) for t in (layer.scales, layer.zeros))
+    return lambda x, pdl=0: torch.ops.matgptq_cuda.matmul_matgptq_zeros(x, packed, s, z, n_out, n_in, b, gs, flag | pdl)
+
+
+@pytest.mark.parametrize("gs,m", [(128, 64), (-1, 40), (32, 130)])
+def test_a_slow_kernel_before_it_in_the_chain(lib, cuda, gs, m):
+    # the product starts while the kernel before it rests, for longer than any of its waits would last: it waits for its
+    # activations all the same and reports nothing
+    product = _zp_layer(2048, 4096, 4, gs, torch.float16, cuda)
+    x = synth.make_activations(m, 4096, seed=m, dtype=torch.float16, device=cuda)
+    want = product(x)
+    late = torch.zeros_like(x)
+    stream = torch.cuda.current_stream().cuda_stream
+    assert lib.matgptq_b200_selftest_late_writer(x.data_ptr(), late.data_ptr(), x.numel(), 2500, stream) == 0
+    y = product(late, pdl=4)
+    assert _native.device_status() == 0
+    assert torch.equal(y, want)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("n,b,gs,m", [(4096, 4, 128, 48),   # K split
+                                      (8192, 8, -1, 200),   # and not
+                                      (2048, 3, 32, 24)])
+def test_chained_products(cuda, dtype, n, b, gs, m):
+    # each product's result is the next one's input, all launched with programmatic dependent launch; a result's memory comes
+    # back two products later, so that one written too early shows as well
+    products = [_zp_layer(n, n, b, gs, dtype, cuda) for _ in range(2)]
+    x = synth.make_activations(m, n, seed=m, dtype=dtype, device=cuda)
+
+    def chain(pdl):
+        y = x
+        for i in range(4):
+            y = products[i & 1](y, pdl)
+        return y
+    want = chain(0)
+    assert want.isfinite().all() and want.abs().max() > 0
+    for _ in range(4):
+        assert torch.equal(chain(4), want)
+    assert _native.device_status() == 0
