@@ -21,7 +21,8 @@
 //
 // The weights are never rounded: scale and zero point act in fp32, as in the GEMV (gemv.cu).  K is split over the CTAs of a
 // thread-block cluster, which add their sums through distributed shared memory in the order of the K ranges.  Every mbarrier
-// wait is bounded; tensor memory is freed on every path.
+// wait is bounded.  A warp that gives up hands nothing on any more, so that the others give up in turn; the issuing warp stays
+// until its copies and MMAs have ended (again with a limit), and tensor memory is freed on every path.
 //
 // The tiles of gemm_tc.cu hold scale * (code - zero) rounded to 16 bits, 1.4 times the error; the GEMV
 // scales in fp32 but takes a pass, with its own decoding, for every 16 rows.  What bounds it: a launch takes about 4 us around
@@ -67,7 +68,7 @@ struct TsParams {
 // Shared memory: barriers (8 bytes each) and the address of the tensor memory, the groups' activation sums, the B stages, the
 // raw stages.
 constexpr int kTsBarFull = 0, kTsBarDone = 8 * kTsMaxStages, kTsBarDEmpty = 16 * kTsMaxStages, kTsBarRawFull = kTsBarDEmpty + 32,
-              kTsTmemSlot = kTsBarRawFull + 8 * kTsRawStages;
+              kTsBarEnd = kTsBarRawFull + 8 * kTsRawStages, kTsTmemSlot = kTsBarEnd + 8;
 constexpr int kTsOffSums = 1024, kTsOffStages = 4096;
 static_assert(kTsTmemSlot + 4 <= kTsOffSums && kTsOffSums + 3 * 4 * kTsMaxCols * 4 <= kTsOffStages, "shared-memory plan");
 
@@ -173,6 +174,7 @@ __global__ void __launch_bounds__(kTsWarps * 32, 1) gemm_ts_kernel(const TsParam
     if (lane < 4) {
       mbar_init(base + kTsBarDEmpty + 8 * lane, scalers);
     }
+    if (lane == 0) mbar_init(base + kTsBarEnd, 1);
     mbar_init_fence();
     __syncwarp();
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(base + kTsTmemSlot) : "memory");
@@ -216,15 +218,18 @@ __global__ void __launch_bounds__(kTsWarps * 32, 1) gemm_ts_kernel(const TsParam
     ring.advance(phase, stages);
     bool ahead = true;  // in the first pass through the stages, which are free from the start
     const uint32_t a_lane = tmem + a_col0 + (static_cast<uint32_t>(quad * 32 + (j & 1) * 16) << 16) + (j >> 1) * 64;
-    for (int kb = phase; kb < my_blocks; kb += step * kAhead) {
+    for (int kb = phase; kb < my_blocks && !failed; kb += step * kAhead) {
 #pragma unroll
       for (int a = 0; a < kAhead; ++a) {
-        if (kb + a * step < my_blocks) {
+        if (kb + a * step < my_blocks && !failed) {
           if (ahead && ring.parity == 0) {
             asm volatile("griddepcontrol.wait;" ::: "memory");
             ahead = false;
           }
-          if (!failed && !mbar_wait_chain(base + kTsBarDone + 8 * ring.idx, ring.parity)) failed = true;
+          if (!mbar_wait_chain(base + kTsBarDone + 8 * ring.idx, ring.parity)) {
+            failed = true;
+            break;
+          }
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           const uint32_t taddr = a_lane + ring.idx * (rbs * 64);
           ts_put_quarter<B, BF16, 0>(wq[a], taddr);
@@ -287,6 +292,7 @@ __global__ void __launch_bounds__(kTsWarps * 32, 1) gemm_ts_kernel(const TsParam
     float *sums = reinterpret_cast<float *>(base_ptr + kTsOffSums);
     auto sum_block = [&](int buf, bool group_ends) {
       if (!failed && !mbar_wait_chain(base + kTsBarFull + 8 * b_ring.idx, b_ring.parity)) failed = true;
+      if (failed) return;
       if (8 * sw < p.ncols) {
         const int g = lane >> 2, t = lane & 3;
         const uint32_t row = base + kTsOffStages + b_ring.idx * b_stage_bytes + (8 * sw + g) * 128;
@@ -333,8 +339,11 @@ __global__ void __launch_bounds__(kTsWarps * 32, 1) gemm_ts_kernel(const TsParam
       asm volatile("bar.sync 1, %0;" ::"n"(kTsScalers * 32) : "memory");  // the sums of block blk are there
       sum_buf = sum_buf == 2 ? 0 : sum_buf + 1;
       if (blk + 1 < nblk) sum_block(GS == -1 ? 0 : sum_buf, GS != -1 || blk + 2 == nblk);
-      if (!scales_any) continue;
-      if (!failed && !mbar_wait_chain(base + kTsBarDone + 8 * done.idx, done.parity)) failed = true;
+      if (!scales_any || failed) continue;  // all eight warps pass every named barrier
+      if (!mbar_wait_chain(base + kTsBarDone + 8 * done.idx, done.parity)) {
+        failed = true;
+        continue;
+      }
       done.advance(1, stages);
       if (GS == -1 && blk + 1 < nblk) continue;  // waited for all the same: a parity tells neighbouring phases apart only
 #pragma unroll
@@ -404,8 +413,11 @@ __global__ void __launch_bounds__(kTsWarps * 32, 1) gemm_ts_kernel(const TsParam
     asm volatile("griddepcontrol.wait;" ::: "memory");
     for (int blk = 0; blk < nblk; ++blk) {
       const int slot = blk & (kTsRawStages - 1);
-      if (!failed && !mbar_wait_chain(base + kTsBarRawFull + 8 * slot, (blk / kTsRawStages) & 1)) failed = true;
-      if (!failed && !mbar_wait_chain(base + kTsBarDone + 8 * ring.idx, ring.parity)) failed = true;
+      if (!mbar_wait_chain(base + kTsBarRawFull + 8 * slot, (blk / kTsRawStages) & 1) ||
+          !mbar_wait_chain(base + kTsBarDone + 8 * ring.idx, ring.parity)) {
+        failed = true;
+        break;
+      }
       uint32_t raw = raw0 + slot * b_stage_bytes, dst = tile0_addr + ring.idx * b_stage_bytes;
       for (int u = 0; u < nunits; ++u) {
         uint4 v[4];
@@ -446,7 +458,8 @@ __global__ void __launch_bounds__(kTsWarps * 32, 1) gemm_ts_kernel(const TsParam
     const uint64_t db0 = umma_smem_desc(base + kTsOffStages, 16, 1024, 2);
     const uint32_t b_stage16 = b_stage_bytes >> 4, b_half16 = b_half_bytes >> 4;
     TsRing ring(0, 0), d_ring(0, 1);
-    for (int blk = 0; blk < nblk; ++blk) {
+    int blk = 0;
+    for (; blk < nblk; ++blk) {
       if (!mbar_wait_chain(base + kTsBarFull + 8 * ring.idx, ring.parity)) {
         failed = true;
         break;
@@ -482,6 +495,13 @@ __global__ void __launch_bounds__(kTsWarps * 32, 1) gemm_ts_kernel(const TsParam
       if (failed) break;
       ring.advance(1, stages);
     }
+    // Nothing of this CTA may be in flight when it frees its memory.  A scaling warp that gave up has not waited for the MMAs,
+    // and where this warp gives up at a block, the activations of that and the following ones may still be on their way.
+    if (elect_one()) umma_commit(base + kTsBarEnd);
+    __syncwarp();
+    if (!mbar_wait_chain(base + kTsBarEnd, 0)) failed = true;
+    for (int i = blk; i < min(nblk, blk + kTsRawStages); ++i)
+      if (!mbar_wait_chain(base + kTsBarRawFull + 8 * (i & (kTsRawStages - 1)), (i / kTsRawStages) & 1)) break;
     if (failed) report_status(kStatusWeightCopyTimeout);
   }
 
