@@ -69,6 +69,15 @@ int matgptq_b200_matmul_zp(int64_t bitwidth, int64_t group_size, int64_t n_out, 
                            const void *w, const void *s, const void *z, const void *x, void *y, void *stream,
                            uint32_t flags);
 
+/* How the tensor-core kernel for zero points lays out a product of more than 16 rows, without launching it (needs no device).
+ * For tuning and tests.
+ *   sm_count, clusters_at_once: the device's SMs and how many clusters of 2, 3, .. 8 CTAs it runs at once (seven values,
+ *                               INT_MAX = unknown);  max_split: CTAs along K at most (1 to 8)
+ *   plan: seven values: batch blocks, columns of one, row tiles of a CTA, CTAs along K, accumulators, stages, bytes of shared
+ *         memory */
+int matgptq_b200_zp_plan(int64_t group_size, int64_t n_out, int64_t n_in, int64_t batch, int sm_count,
+                         const int *clusters_at_once, int max_split, int *plan);
+
 /* Same, with the launch shape of the GEMV forced (0 = choose).  For tuning and tests.
  *   warps_per_cta: low byte = warps per CTA (1..16); next byte = how many of them share one row tile and split
  *                  the CTA's K range between them (0 or 1 = none; must divide the warps; needs the CTA's whole K

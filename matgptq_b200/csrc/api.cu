@@ -128,6 +128,20 @@ int matgptq_b200_matmul_zp(int64_t bitwidth, int64_t group_size, int64_t n_out, 
   return matmul_impl(bitwidth, group_size, n_out, n_in, batch, w, s, x, y, stream, flags, nullptr, 0, 0, 0, 0, z);
 }
 
+int matgptq_b200_zp_plan(int64_t group_size, int64_t n_out, int64_t n_in, int64_t batch, int sm_count,
+                         const int *clusters_at_once, int max_split, int *plan) {
+  const int st = check_shape(n_out, n_in, 8, group_size);
+  if (st != MG_OK) return st;
+  if (batch <= 16 || batch > (1 << 24) || sm_count < 1 || !clusters_at_once || max_split < 1 || max_split > 8 || !plan) return MG_ERR_BAD_ARG;
+  for (int i = 0; i < 7; ++i)
+    if (clusters_at_once[i] < 1) return MG_ERR_BAD_ARG;
+  const mg::TsPlan p = mg::gemm_ts_plan(static_cast<int>(n_out), static_cast<int>(n_in), static_cast<int>(batch),
+                                        static_cast<int>(group_size), max_split, sm_count, clusters_at_once);
+  const int out[7] = {p.blocks, p.ncols, p.tiles, p.split, p.accumulators, p.stages, p.smem};
+  for (int i = 0; i < 7; ++i) plan[i] = out[i];
+  return MG_OK;
+}
+
 int matgptq_b200_matmul_ws(int64_t bitwidth, int64_t group_size, int64_t n_out, int64_t n_in, int64_t batch,
                            const void *w, const void *s, const void *x, void *y, void *stream, uint32_t flags,
                            void *workspace, int64_t workspace_bytes, int path, int split_k) {

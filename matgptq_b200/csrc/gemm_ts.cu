@@ -554,15 +554,11 @@ __global__ void __launch_bounds__(kTsWarps * 32, 1) gemm_ts_kernel(const TsParam
 // ----------------------------------------------------------------------------
 // host side
 // ----------------------------------------------------------------------------
-struct TsPlan {
-  int blocks, ncols, tiles, split, accumulators, stages, smem;
-};
-
 // Batch blocks of at most 64 rows; 4, 8 or 16 row tiles a CTA (16 with at most 32 rows: a scaling warp holds 32 sums a lane).
-// Among these and the K splits the cheapest by what a block of 128 in-features, a launch and a reduction were measured to
-// take on B200 (microseconds, 16 to 64 rows: 8 tiles 0.34 to 0.50, 16 tiles 0.59 to 0.62; with zero points the sums of the
-// activations add to that).
-static TsPlan ts_plan(int N, int K, int M, int group_size, int sm_count) {
+// Among these and the K splits up to `max_split` the cheapest by what a block of 128 in-features, a launch and a reduction were
+// measured to take on B200 (microseconds, 16 to 64 rows: 8 tiles 0.34 to 0.50, 16 tiles 0.59 to 0.62; with zero points the sums
+// of the activations add to that).
+TsPlan gemm_ts_plan(int N, int K, int M, int group_size, int max_split, int sm_count, const int *clusters_at_once) {
   TsPlan best = {};
   best.blocks = (M + kTsMaxCols - 1) / kTsMaxCols;
   const int rows = (M + best.blocks - 1) / best.blocks;
@@ -570,12 +566,12 @@ static TsPlan ts_plan(int N, int K, int M, int group_size, int sm_count) {
   const int tiles16 = N / 16, kblocks = K / 128;
   float best_cost = 1e30f;
   for (int rt = 4; rt <= (best.ncols <= 32 ? 16 : 8); rt *= 2) {
-    const int clusters = (tiles16 + rt - 1) / rt * best.blocks;
+    const long long clusters = static_cast<long long>((tiles16 + rt - 1) / rt) * best.blocks;
     float block = (rt == 4 ? 0.30f : rt == 8 ? 0.36f : 0.60f) + 0.0035f * (best.ncols - 16);
     if (group_size == 32) block *= 2.f;
-    for (int split = 1; split <= 8 && split <= kblocks; ++split) {
-      const int at_once = split > 1 ? tc_clusters_at_once(split) : sm_count;
-      const int waves = (clusters + at_once - 1) / at_once;
+    for (int split = 1; split <= max_split && split <= kblocks; ++split) {
+      const int at_once = split == 1 ? sm_count : clusters_at_once ? clusters_at_once[split - 2] : tc_clusters_at_once(split);
+      const float waves = static_cast<float>((clusters - 1) / at_once + 1);  // at_once may be INT_MAX
       const float cost = waves * (4.f + (kblocks + split - 1) / split * block) + (split > 1 ? 2.5f + 0.02f * best.ncols : 0.f);
       if (cost < best_cost) {
         best_cost = cost;
@@ -655,7 +651,6 @@ int gemm_ts_launch(int bitwidth, int group_size, int N, int K, int M, const void
     const int st = current_device_sm_count(&sm_count);
     if (st != MG_OK) return st;
   }
-  TsPlan plan = ts_plan(N, K, M, group_size, sm_count);
   TsParams p;
   p.w = static_cast<const uint32_t *>(w);
   p.s = static_cast<const uint16_t *>(s);
@@ -667,16 +662,20 @@ int gemm_ts_launch(int bitwidth, int group_size, int N, int K, int M, const void
   p.M = M;
   p.ldy = ldy > 0 ? ldy : N;
   p.kblocks = K / 128;
-  p.split = plan.split;
-  p.tiles = plan.tiles;
-  p.ncols = plan.ncols;
-  p.accumulators = plan.accumulators;
-  p.stages = plan.stages;
-  int r = launch_ts_bits(p, plan, bitwidth, group_size, bf16, stream, pdl);
-  if (r == MG_ERR_CUDA && plan.split > 1) {  // a device that cannot place the cluster (a partitioned GPU, say): nothing was launched
+  const auto launch = [&](int max_split, int *split) {
+    const TsPlan plan = gemm_ts_plan(N, K, M, group_size, max_split, sm_count, nullptr);
+    *split = p.split = plan.split;
+    p.tiles = plan.tiles;
+    p.ncols = plan.ncols;
+    p.accumulators = plan.accumulators;
+    p.stages = plan.stages;
+    return launch_ts_bits(p, plan, bitwidth, group_size, bf16, stream, pdl);
+  };
+  int split = 1;
+  int r = launch(8, &split);
+  if (r == MG_ERR_CUDA && split > 1) {  // a device that cannot place the cluster (a partitioned GPU, say): nothing was launched
     (void)cudaGetLastError();
-    p.split = plan.split = 1;
-    r = launch_ts_bits(p, plan, bitwidth, group_size, bf16, stream, pdl);
+    r = launch(1, &split);  // with the tiles and stages of a launch without clusters
   }
   return r;
 }

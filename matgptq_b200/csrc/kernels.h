@@ -70,6 +70,14 @@ int tc_clusters_at_once(int size);
 // gemm_ts.cu
 int gemm_ts_launch(int bitwidth, int group_size, int N, int K, int M, const void *w, const void *s, const void *z, const void *x,
                    void *y, bool bf16, bool pdl, cudaStream_t stream, int ldy = 0);
+struct TsPlan {
+  int blocks, ncols;  // batch blocks, columns of one (a multiple of 16)
+  int tiles, split;   // row tiles of a CTA, CTAs along K
+  int accumulators, stages, smem;
+};
+// How a product is laid out on a device with sm_count SMs that runs clusters_at_once[0..6] clusters of 2 to 8 CTAs at once
+// (null: the current device), with at most max_split CTAs along K.
+TsPlan gemm_ts_plan(int N, int K, int M, int group_size, int max_split, int sm_count, const int *clusters_at_once);
 int gemm_ts_device_status(int *status_out, int reset);
 
 // selftest.cu
