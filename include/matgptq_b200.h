@@ -63,19 +63,22 @@ int matgptq_b200_matmul(int64_t bitwidth, int64_t group_size, int64_t n_out, int
  * product with per-group zero points, Wdq = s * (code * 2^(8-b) - zero), the formula of dequantize()
  * (src/quant_utils_matgpqt.py:19-22).  `z` holds the zero points in master (8-bit) units, in the type of the
  * scales and in their reordered layout (matgptq_b200_reorder_scales on the [N, G] zero points).  z == NULL is
- * matgptq_b200_matmul.  Every batch size runs on the GEMV family (more than 16 rows in passes of 16).
+ * matgptq_b200_matmul.  Up to 16 rows, and above as long as its passes of 16 rows run side by side (narrow layers), the
+ * product runs on the GEMV, otherwise on the tensor cores (tcgen05).  Neither rounds the weights to 16 bits: scale and
+ * zero point act in fp32.  With FLAG_BF16 the GEMV takes activations of up to 65504 in magnitude, as
+ * matgptq_b200_matmul does on it (what is larger, infinite or NaN counts as a number of that magnitude); the tensor cores take all of bf16.
  */
 int matgptq_b200_matmul_zp(int64_t bitwidth, int64_t group_size, int64_t n_out, int64_t n_in, int64_t batch,
                            const void *w, const void *s, const void *z, const void *x, void *y, void *stream,
                            uint32_t flags);
 
-/* How the tensor-core kernel for zero points lays out a product of more than 16 rows, without launching it (needs no device).
+/* The path of a product with zero points and how the tensor-core kernel lays it out, without launching it (needs no device).
  * For tuning and tests.
  *   sm_count, clusters_at_once: the device's SMs and how many clusters of 2, 3, .. 8 CTAs it runs at once (seven values,
  *                               INT_MAX = unknown);  max_split: CTAs along K at most (1 to 8)
- *   plan: seven values: batch blocks, columns of one, row tiles of a CTA, CTAs along K, accumulators, stages, bytes of shared
- *         memory */
-int matgptq_b200_zp_plan(int64_t group_size, int64_t n_out, int64_t n_in, int64_t batch, int sm_count,
+ *   plan: eight values: path (1 = GEMV, 2 = tensor cores), then for the tensor cores, also where they are not chosen, batch
+ *         blocks, columns of one, row tiles of a CTA, CTAs along K, accumulators, stages, bytes of shared memory */
+int matgptq_b200_zp_plan(int64_t bitwidth, int64_t group_size, int64_t n_out, int64_t n_in, int64_t batch, int sm_count,
                          const int *clusters_at_once, int max_split, int *plan);
 
 /* Same, with the launch shape of the GEMV forced (0 = choose).  For tuning and tests.

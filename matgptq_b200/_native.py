@@ -61,7 +61,7 @@ SIGNATURES = {
     "matgptq_b200_reorder_scales_host": (_c_int, [_c_ptr, _c_ptr, _c_i64, _c_i64, _c_i64]),
     "matgptq_b200_device_status": (_c_int, [ctypes.POINTER(ctypes.c_int), _c_int]),
     "matgptq_b200_selftest_wait_timeout": (_c_int, [_c_int, _c_ptr, _c_ptr]),
-    "matgptq_b200_zp_plan": (_c_int, [_c_i64, _c_i64, _c_i64, _c_i64, _c_int, _c_ptr, _c_int, _c_ptr]),
+    "matgptq_b200_zp_plan": (_c_int, [_c_i64] * 5 + [_c_int, _c_ptr, _c_int, _c_ptr]),
     "matgptq_b200_selftest_late_writer": (_c_int, [_c_ptr, _c_ptr, _c_i64, _c_int, _c_ptr]),
     "matgptq_b200_dequantize": (_c_int, [_c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_i64, _c_i64, _c_int, _c_i64, _c_u32, _c_ptr]),
 }

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include "../../include/matgptq_b200.h"
+#include "host_util.h"
 #include "kernels.h"
 
 namespace {
@@ -60,6 +61,24 @@ static bool uses_tensor_cores(int64_t n_out, int64_t batch) {
   return batch > 24;
 }
 
+// The same choice with zero points: the GEMV up to 16 rows and, above, as long as its passes of 16 rows run side by side, then
+// the tensor-core path that scales in fp32 (gemm_ts.cu), which like the GEMV rounds no weight to 16 bits.  Measured on B200
+// (K = 4096, 4 bits, group 128, fp16, cold weights, GEMV against tensor cores in us):
+//   256 out-features: 17 rows 3.9 / 6.6, 64 rows 4.3 / 8.5, 128 rows 6.3 / 9.2, 256 rows (two waves of CTAs) 11.4 / 9.7
+//   1024:             17 rows 5.2 / 7.7, 32 rows 5.8 / 7.9, 48 rows (two waves) 9.7 / 8.7
+//   2048 and 4096:    two waves at 17 rows already, 9.8 / 10.2 and 11.8 / 12.6; 32 rows 11.3 / 10.3 and 13.2 / 12.7
+// With groups of 32 the tensor cores are further behind (1024: 32 rows 7.1 / 9.8); with one scale per row, where a CTA scales
+// once, they are ahead also of a single wave that stages its activations in pieces (512 x 14336, 32 rows 12.9 / 10.9) or has
+// only a few blocks of in-features to multiply (4096 x 256, 32 rows 5.1 / 3.7).
+static bool zp_uses_tensor_cores(int64_t bitwidth, int64_t group_size, int64_t n_out, int64_t n_in, int64_t batch, int sm_count) {
+  if (batch <= 16) return false;
+  bool whole = false;
+  if (!mg::gemv_zp_in_one_wave(static_cast<int>(bitwidth), static_cast<int>(group_size), static_cast<int>(n_out),
+                               static_cast<int>(n_in), static_cast<int>(batch), sm_count, &whole))
+    return true;
+  return group_size == -1 && (!whole || n_in < 512);
+}
+
 static int sm_count_of_current_device(int *out) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return MG_ERR_CUDA;
@@ -84,11 +103,10 @@ static int matmul_impl(int64_t bitwidth, int64_t group_size, int64_t n_out, int6
   const bool tensor_core = path == 2 || (path == 0 && uses_tensor_cores(n_out, batch));
   int r;
   if (z) {
-    // Zero points: the GEMV up to 16 rows, then the tensor-core path that scales in fp32 (gemm_ts.cu), which like the GEMV
-    // rounds no weight to 16 bits.  16 rows are one pass of the GEMV; at 17 it reads and decodes the weights twice.
-    // 4096 x 4096, 4 bits, GEMV against tensor cores in us: 16 rows 8.2 / 11.4, 32 rows 16.2 / 12.3, 128 rows 58.1 / 21.9.
     if (path > 1) return MG_ERR_UNSUPPORTED;
-    if (path == 0 && batch > 16)
+    int sms = 0;
+    if (batch > 16 && mg::current_device_sm_count(&sms) != MG_OK) return MG_ERR_CUDA;
+    if (path == 0 && zp_uses_tensor_cores(bitwidth, group_size, n_out, n_in, batch, sms))
       r = mg::gemm_ts_launch(static_cast<int>(bitwidth), static_cast<int>(group_size), static_cast<int>(n_out), static_cast<int>(n_in),
                              static_cast<int>(batch), w, s, z, x, y, bf16, pdl, cs);
     else
@@ -128,17 +146,18 @@ int matgptq_b200_matmul_zp(int64_t bitwidth, int64_t group_size, int64_t n_out, 
   return matmul_impl(bitwidth, group_size, n_out, n_in, batch, w, s, x, y, stream, flags, nullptr, 0, 0, 0, 0, z);
 }
 
-int matgptq_b200_zp_plan(int64_t group_size, int64_t n_out, int64_t n_in, int64_t batch, int sm_count,
+int matgptq_b200_zp_plan(int64_t bitwidth, int64_t group_size, int64_t n_out, int64_t n_in, int64_t batch, int sm_count,
                          const int *clusters_at_once, int max_split, int *plan) {
-  const int st = check_shape(n_out, n_in, 8, group_size);
+  const int st = check_shape(n_out, n_in, bitwidth, group_size);
   if (st != MG_OK) return st;
-  if (batch <= 16 || batch > (1 << 24) || sm_count < 1 || !clusters_at_once || max_split < 1 || max_split > 8 || !plan) return MG_ERR_BAD_ARG;
+  if (batch < 1 || batch > (1 << 24) || sm_count < 1 || !clusters_at_once || max_split < 1 || max_split > 8 || !plan) return MG_ERR_BAD_ARG;
   for (int i = 0; i < 7; ++i)
     if (clusters_at_once[i] < 1) return MG_ERR_BAD_ARG;
   const mg::TsPlan p = mg::gemm_ts_plan(static_cast<int>(n_out), static_cast<int>(n_in), static_cast<int>(batch),
                                         static_cast<int>(group_size), max_split, sm_count, clusters_at_once);
-  const int out[7] = {p.blocks, p.ncols, p.tiles, p.split, p.accumulators, p.stages, p.smem};
-  for (int i = 0; i < 7; ++i) plan[i] = out[i];
+  const int path = zp_uses_tensor_cores(bitwidth, group_size, n_out, n_in, batch, sm_count) ? 2 : 1;
+  const int out[8] = {path, p.blocks, p.ncols, p.tiles, p.split, p.accumulators, p.stages, p.smem};
+  for (int i = 0; i < 8; ++i) plan[i] = out[i];
   return MG_OK;
 }
 

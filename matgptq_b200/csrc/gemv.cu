@@ -733,11 +733,14 @@ __global__ void __launch_bounds__(512, 1) gemv_grouped_kernel(const GroupedParam
 // Shared memory per CTA that leaves room for exactly `ctas` CTAs on an SM (227 KB usable, 1 KB reserved per CTA).
 static inline int smem_for_ctas_per_sm(int ctas) { return (227 * 1024) / ctas - 1024; }
 
-template <int B, int GS, bool BF16, int NT>
-static int launch_gemv(GemvParams p, int R, cudaStream_t stream, bool pdl) {
-  auto kernel = gemv_kernel<B, GS, BF16, NT, kZP>;
-  const int S = p.split;
-  const int max_nblk = (p.kblocks + S - 1) / S;
+// What a CTA of R warps takes of its SM's shared memory.
+struct GemvFit {
+  int xblocks, stages;
+  bool whole;  // the CTA's K slice of the activations is staged in one piece
+  size_t smem;
+};
+
+template <int B, int GS, int NT> static int gemv_fit(int R, int kslices, int M, int max_nblk, GemvFit *fit) {
   // About 16 warps per SM: CTAs of R warps come 16/R to an SM.  The ring takes what is left of that share of
   // the shared memory after the activations (2 to 8 stages), and the request is padded so that one CTA more
   // does not fit: the block scheduler otherwise stacks CTAs on the SMs that free up first.
@@ -747,19 +750,32 @@ static int launch_gemv(GemvParams p, int R, cudaStream_t stream, bool pdl) {
   // Activations: the whole K slice of the CTA in one piece when that leaves room for two ring stages (no
   // buffer turnover, so the warps never meet at a barrier inside the loop), else double-buffered stages.
   int xblocks = max_nblk;
-  if (make_plan<B, GS, NT, kZP>(R, p.M, max_nblk, 2, xblocks).total > budget) {
-    if (p.kslices > 1) return MG_ERR_UNSUPPORTED;  // K slices inside a CTA need the whole slice of the activations staged
+  if (make_plan<B, GS, NT, kZP>(R, M, max_nblk, 2, xblocks).total > budget) {
+    if (kslices > 1) return MG_ERR_UNSUPPORTED;  // K slices inside a CTA need the whole slice of the activations staged
     xblocks = (NT == 1) ? 8 : 4;
   }
   if (xblocks > max_nblk) xblocks = max_nblk;
   int stages = 2;
-  while (stages < 8 && stages < nchunks && make_plan<B, GS, NT, kZP>(R, p.M, max_nblk, stages + 1, xblocks).total <= budget) ++stages;
-  p.stages = stages;
-  p.xblocks = xblocks;
-  const SmemPlan plan = make_plan<B, GS, NT, kZP>(R, p.M, max_nblk, stages, xblocks);
+  while (stages < 8 && stages < nchunks && make_plan<B, GS, NT, kZP>(R, M, max_nblk, stages + 1, xblocks).total <= budget) ++stages;
+  const SmemPlan plan = make_plan<B, GS, NT, kZP>(R, M, max_nblk, stages, xblocks);
   if (plan.total > 227 * 1024 - 1024) return MG_ERR_UNSUPPORTED;
   const int floor_bytes = smem_for_ctas_per_sm(ctas_per_sm + 1) + 1;
-  const size_t smem = static_cast<size_t>(plan.total > floor_bytes ? plan.total : floor_bytes);
+  *fit = GemvFit{xblocks, stages, xblocks == max_nblk, static_cast<size_t>(plan.total > floor_bytes ? plan.total : floor_bytes)};
+  return MG_OK;
+}
+
+template <int B, int GS, bool BF16, int NT>
+static int launch_gemv(GemvParams p, int R, cudaStream_t stream, bool pdl) {
+  auto kernel = gemv_kernel<B, GS, BF16, NT, kZP>;
+  const int S = p.split;
+  GemvFit fit;
+  {
+    const int st = gemv_fit<B, GS, NT>(R, p.kslices, p.M, (p.kblocks + S - 1) / S, &fit);
+    if (st != MG_OK) return st;
+  }
+  p.stages = fit.stages;
+  p.xblocks = fit.xblocks;
+  const size_t smem = fit.smem;
   if (smem > 48 * 1024) {
     static SharedMemoryOptIn opt_in;  // one per instantiation of this launcher
     const int st = opt_in.ensure(kernel, 226 * 1024);
@@ -843,6 +859,45 @@ static void gemv_pick_config(int tiles, int kblocks, int batch, int sm_count, Ge
     *first = GemvShape{16, 1, 2};
   }
 }
+
+#if MG_GEMV_ZP
+template <int B> static int gemv_fit_group(int group_size, const GemvShape &c, int M, int kblocks, GemvFit *fit) {
+  const int max_nblk = (kblocks + c.S - 1) / c.S;
+  if (group_size == 32) return gemv_fit<B, 32, 2>(c.R, c.RK, M, max_nblk, fit);
+  if (group_size == 128) return gemv_fit<B, 128, 2>(c.R, c.RK, M, max_nblk, fit);
+  return gemv_fit<B, -1, 2>(c.R, c.RK, M, max_nblk, fit);
+}
+
+static int gemv_fit_bits(int bitwidth, int group_size, const GemvShape &c, int M, int kblocks, GemvFit *fit) {
+  switch (bitwidth) {
+    case 2: return gemv_fit_group<2>(group_size, c, M, kblocks, fit);
+    case 3: return gemv_fit_group<3>(group_size, c, M, kblocks, fit);
+    case 4: return gemv_fit_group<4>(group_size, c, M, kblocks, fit);
+    case 6: return gemv_fit_group<6>(group_size, c, M, kblocks, fit);
+    case 8: return gemv_fit_group<8>(group_size, c, M, kblocks, fit);
+    default: return MG_ERR_BAD_ARG;
+  }
+}
+
+// Whether all passes of a product of more than 16 rows run side by side.  The passes are CTAs of their own: on a narrow layer a
+// few of them leave SMs idle, and more passes cost next to nothing until the slots of the SMs are taken.  Not counted as free:
+// the last 5 % of the slots, which clusters do not fill (1536 x 1024 at 48 rows: 288 CTAs of 296, 8.0 us, 4.7 at 32 rows), and
+// more than eight CTAs on an SM (1536 x 256: 96 rows, 1152 CTAs 5.0 us, 128 rows, 1536 CTAs 8.6).
+bool gemv_zp_in_one_wave(int bitwidth, int group_size, int N, int K, int M, int sm_count, bool *whole) {
+  GemvShape c, second;
+  gemv_pick_config(N / 16, K / 128, 16, sm_count, &c, &second);
+  GemvFit fit;
+  if (gemv_fit_bits(bitwidth, group_size, c, M, K / 128, &fit) != MG_OK) {
+    c = second;
+    if (gemv_fit_bits(bitwidth, group_size, c, M, K / 128, &fit) != MG_OK) return false;
+  }
+  *whole = fit.whole;
+  const int Rt = c.R / c.RK;
+  const long long ctas = static_cast<long long>((N / 16 + Rt - 1) / Rt) * c.S * ((M + 15) / 16);
+  const int per_sm = static_cast<int>(227 * 1024 / (fit.smem + 1024));
+  return ctas * 20 <= 19ll * (per_sm < 8 ? per_sm : 8) * sm_count;
+}
+#endif
 
 static int launch_shape(GemvParams p, const GemvShape &c, int bitwidth, int group_size, bool bf16, bool pdl,
                         cudaStream_t stream) {

@@ -53,6 +53,10 @@ struct GroupedSegment {
 int gemv_grouped_launch(const GroupedSegment *segments, int nseg, int group_size, int K, int M, const void *x, void *y,
                         int ldy, bool bf16, bool pdl, cudaStream_t stream);
 
+// Whether the passes of a product with zero points of more than 16 rows fit on the device at once; *whole: a CTA stages its
+// activations in one piece.
+bool gemv_zp_in_one_wave(int bitwidth, int group_size, int N, int K, int M, int sm_count, bool *whole);
+
 int gemv_device_status(int *status_out, int reset);
 int gemv_zp_device_status(int *status_out, int reset);
 

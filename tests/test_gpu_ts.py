@@ -1,5 +1,7 @@
 """Tensor-core path with the weights in tensor memory and fp32 scaling: edges of its row tiles, batch blocks, stages and K
 splits, against the unrounded weights in 64 bits."""
+import ctypes
+
 import pytest
 import torch
 
@@ -82,4 +84,50 @@ def test_chained_products(cuda, dtype, n, b, gs, m):
     assert want.isfinite().all() and want.abs().max() > 0
     for _ in range(4):
         assert torch.equal(chain(4), want)
+    assert _native.device_status() == 0
+
+
+def _path(lib, b, gs, n, k, m):
+    plan = (ctypes.c_int * 8)()
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert lib.matgptq_b200_zp_plan(b, gs, n, k, m, sms, (ctypes.c_int * 7)(*[sms // s for s in range(2, 9)]), 8, plan) == 0
+    return plan[0]
+
+
+@pytest.mark.parametrize("b", (2, 3, 4, 6, 8))
+@pytest.mark.parametrize("gs", [-1, 32, 128])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_weights_read_back_on_the_tensor_cores(lib, cuda, b, gs, dtype):
+    # one-hot rows give the weights, rounded once, of a layer wide enough for the tensor cores
+    n_out, n_in = 4112, 512
+    assert _path(lib, b, gs, n_out, n_in, n_in) == 2
+    layer = synth.make_layer(n_out, n_in, gs, seed=b, sym=False, dtype=dtype, device=cuda)
+    flag = 1 | (2 if dtype == torch.bfloat16 else 0)
+    layer.zeros[::7] = 0.0
+    layer.zeros[3::7] = 255.0
+    packed = torch.ops.matgptq_cuda.slice_pack_matgptq_qweights(layer.qweight, n_out, n_in, 8, b, gs, flag)
+    s, z = (torch.ops.matgptq_cuda.reorder_matgptq_scales(t, n_out, n_in, gs) for t in (layer.scales, layer.zeros))
+    want = oracle.dequantize_weight(layer.qweight.cpu(), layer.scales.cpu(), layer.zeros.cpu(), 8, b)
+    y = torch.ops.matgptq_cuda.matmul_matgptq_zeros(torch.eye(n_in, dtype=dtype, device=cuda), packed, s, z, n_out, n_in, b, gs, flag)
+    assert _native.device_status() == 0
+    assert torch.equal(y.cpu(), want.t().contiguous())
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("b,gs,n,k", [(4, 128, 256, 4096), (8, 32, 1024, 1024), (3, -1, 528, 2944)])
+def test_both_sides_of_the_dispatch(lib, cuda, dtype, b, gs, n, k):
+    # the last batch on the GEMV, in several passes with a ragged one, and the first on the tensor cores
+    rows = [m for m in range(17, 600) if _path(lib, b, gs, n, k, m) == 1][-1]
+    product = _zp_layer(n, k, b, gs, dtype, cuda)
+    layer = synth.make_layer(n, k, gs, seed=b, sym=False, dtype=dtype, device=cuda)
+    group = k if gs == -1 else gs
+    codes = oracle.matryoshka_slice(layer.qweight, 8, b).double() * 2 ** (8 - b) - 128
+    scale, zero = (t.double().repeat_interleave(group, 1) for t in (layer.scales, layer.zeros))
+    for m in (rows - 15, rows, rows + 1):
+        x = synth.make_activations(m, k, seed=m, dtype=dtype, device=cuda)
+        ref = x.double() @ (scale * (codes - (zero - 128))).t()
+        # the result is rounded once; sums of the integers and of the activations meet in fp32
+        size = x.double().abs() @ (scale.abs() * (codes.abs() + (zero - 128).abs())).t()
+        half_ulp = 2.0 ** (-8 if dtype == torch.bfloat16 else -11)
+        assert ((product(x).double() - ref).abs() <= half_ulp * ref.abs() * 1.01 + 2.0 ** -19 * size).all(), m
     assert _native.device_status() == 0
