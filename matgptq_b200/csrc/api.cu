@@ -102,16 +102,15 @@ static int matmul_impl(int64_t bitwidth, int64_t group_size, int64_t n_out, int6
   const bool pdl = (flags & MATGPTQ_B200_FLAG_PDL) != 0;
   const bool tensor_core = path == 2 || (path == 0 && uses_tensor_cores(n_out, batch));
   int r;
-  if (z) {
-    if (path > 1) return MG_ERR_UNSUPPORTED;
+  if (z) {  // called with path 0 and no forced shape
     int sms = 0;
     if (batch > 16 && mg::current_device_sm_count(&sms) != MG_OK) return MG_ERR_CUDA;
-    if (path == 0 && zp_uses_tensor_cores(bitwidth, group_size, n_out, n_in, batch, sms))
+    if (zp_uses_tensor_cores(bitwidth, group_size, n_out, n_in, batch, sms))
       r = mg::gemm_ts_launch(static_cast<int>(bitwidth), static_cast<int>(group_size), static_cast<int>(n_out), static_cast<int>(n_in),
                              static_cast<int>(batch), w, s, z, x, y, bf16, pdl, cs);
     else
       r = mg::gemv_zp_launch(static_cast<int>(bitwidth), static_cast<int>(group_size), static_cast<int>(n_out),
-                           static_cast<int>(n_in), static_cast<int>(batch), w, s, z, x, y, bf16, pdl, warps_per_cta, split_k, cs);
+                             static_cast<int>(n_in), static_cast<int>(batch), w, s, z, x, y, bf16, pdl, 0, 0, cs);
   } else if (tensor_core) {
     r = mg::gemm_tc_launch(static_cast<int>(bitwidth), static_cast<int>(group_size), static_cast<int>(n_out),
                            static_cast<int>(n_in), static_cast<int>(batch), w, s, x, y, workspace, workspace_bytes, bf16,

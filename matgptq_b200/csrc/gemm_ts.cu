@@ -56,7 +56,6 @@ struct TsParams {
   const uint16_t *x;
   uint16_t *y;
   int N, K, M;
-  int ldy;
   int kblocks;   // K / 128
   int split;     // CTAs along K
   int tiles;     // row tiles of a CTA: 4, 8 or 16 (16 with at most 32 batch rows)
@@ -394,7 +393,7 @@ __global__ void __launch_bounds__(kTsWarps * 32, 1) gemm_ts_kernel(const TsParam
           if (p.split > 1)
             staging[m * slots + rb * 128 + quad * 32 + lane] = v;
           else if (m < mrows)
-            p.y[static_cast<size_t>(m0 + m) * p.ldy + n] = to_out16<BF16>(v);
+            p.y[static_cast<size_t>(m0 + m) * p.N + n] = to_out16<BF16>(v);
         }
       }
     }
@@ -530,7 +529,7 @@ __global__ void __launch_bounds__(kTsWarps * 32, 1) gemm_ts_kernel(const TsParam
             sum.z = (sum.z + a.z) + b.z;
             sum.w = (sum.w + a.w) + b.w;
           }
-          uint16_t *dst = p.y + static_cast<size_t>(m0 + c_lo + c) * p.ldy + (tile0 + tile) * 16 + (slot & 15);
+          uint16_t *dst = p.y + static_cast<size_t>(m0 + c_lo + c) * p.N + (tile0 + tile) * 16 + (slot & 15);
           const uint16_t o0 = to_out16<BF16>(sum.x), o1 = to_out16<BF16>(sum.y), o2 = to_out16<BF16>(sum.z), o3 = to_out16<BF16>(sum.w);
           if ((reinterpret_cast<uintptr_t>(dst) & 7u) == 0) {
             *reinterpret_cast<uint2 *>(dst) = make_uint2(o0 | (static_cast<uint32_t>(o1) << 16), o2 | (static_cast<uint32_t>(o3) << 16));
@@ -664,7 +663,7 @@ static int launch_ts_bits(const TsParams &p, const TsPlan &plan, int bitwidth, i
 }
 
 int gemm_ts_launch(int bitwidth, int group_size, int N, int K, int M, const void *w, const void *s, const void *z, const void *x,
-                   void *y, bool bf16, bool pdl, cudaStream_t stream, int ldy) {
+                   void *y, bool bf16, bool pdl, cudaStream_t stream) {
   int sm_count = 0;
   {
     const int st = current_device_sm_count(&sm_count);
@@ -679,7 +678,6 @@ int gemm_ts_launch(int bitwidth, int group_size, int N, int K, int M, const void
   p.N = N;
   p.K = K;
   p.M = M;
-  p.ldy = ldy > 0 ? ldy : N;
   p.kblocks = K / 128;
   const auto launch = [&](int max_split, int *split) {
     const TsPlan plan = gemm_ts_plan(N, K, M, group_size, max_split, sm_count, nullptr);

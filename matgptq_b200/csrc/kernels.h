@@ -73,7 +73,7 @@ int tc_clusters_at_once(int size);
 
 // gemm_ts.cu
 int gemm_ts_launch(int bitwidth, int group_size, int N, int K, int M, const void *w, const void *s, const void *z, const void *x,
-                   void *y, bool bf16, bool pdl, cudaStream_t stream, int ldy = 0);
+                   void *y, bool bf16, bool pdl, cudaStream_t stream);
 struct TsPlan {
   int blocks, ncols;  // batch blocks, columns of one (a multiple of 16)
   int tiles, split;   // row tiles of a CTA, CTAs along K
