@@ -131,3 +131,44 @@ def test_both_sides_of_the_dispatch(lib, cuda, dtype, b, gs, n, k):
         half_ulp = 2.0 ** (-8 if dtype == torch.bfloat16 else -11)
         assert ((product(x).double() - ref).abs() <= half_ulp * ref.abs() * 1.01 + 2.0 ** -19 * size).all(), m
     assert _native.device_status() == 0
+
+
+@pytest.mark.parametrize("gs,n,k,m", [(128, 4096, 4096, 40), (-1, 8192, 256, 40)])  # K split, and not
+def test_output_at_any_two_byte_address(lib, cuda, gs, n, k, m):
+    assert _path(lib, 4, gs, n, k, m) == 2
+    layer = synth.make_layer(n, k, gs, seed=1, sym=False, dtype=torch.float16, device=cuda)
+    packed = torch.ops.matgptq_cuda.slice_pack_matgptq_qweights(layer.qweight, n, k, 8, 4, gs, 1)
+    s, z = (torch.ops.matgptq_cuda.reorder_matgptq_scales(t, n, k, gs) for t in (layer.scales, layer.zeros))
+    x = synth.make_activations(m, k, seed=1, dtype=torch.float16, device=cuda)
+    want = torch.ops.matgptq_cuda.matmul_matgptq_zeros(x, packed, s, z, n, k, 4, gs, 1)
+    for shift in range(1, 8):
+        room = torch.full((m * n + 16,), 7.0, dtype=torch.float16, device=cuda)
+        y = room[shift:shift + m * n]
+        assert lib.matgptq_b200_matmul_zp(4, gs, n, k, m, packed.data_ptr(), s.data_ptr(), z.data_ptr(), x.data_ptr(), y.data_ptr(),
+                                          torch.cuda.current_stream().cuda_stream, 1) == 0
+        assert torch.equal(y.view(m, n), want)
+        assert (room[:shift] == 7.0).all() and (room[shift + m * n:] == 7.0).all()
+    assert _native.device_status() == 0
+
+
+@pytest.mark.parametrize("gs", [-1, 32, 128])
+def test_bf16_activations_beyond_the_range_of_fp16(lib, cuda, gs):
+    n, k, m, bf16 = 4096, 1024, 64, torch.bfloat16
+    assert _path(lib, 4, gs, n, k, m) == 2
+    product = _zp_layer(n, k, 4, gs, bf16, cuda)
+    x = synth.make_activations(m, k, seed=3, dtype=bf16, device=cuda)
+    big = (x.float() * 1e6).to(bf16)
+    # a power of two more in the activations is one more in the result
+    assert torch.equal(product((x.float() * 2.0 ** 20).to(bf16)).float(), product(x).float() * 2.0 ** 20)
+    assert (big.abs() > 65504).any() and product(big).isfinite().all()
+    # what is not finite stays in its row
+    odd = x.clone()
+    odd[5, 100], odd[9, 7], odd[63, 1023] = float("inf"), float("nan"), float("-inf")
+    y, others = product(odd), [r for r in range(m) if r not in (5, 9, 63)]
+    assert not y[[5, 9, 63]].isfinite().any()
+    assert torch.equal(y[others], product(x)[others])
+    # the GEMV's limit: what is larger counts as 65504
+    small = _zp_layer(256, k, 4, gs, bf16, cuda)
+    assert _path(lib, 4, gs, 256, k, 16) == 1
+    assert torch.equal(small(big[:16]), small(big[:16].clamp(-65504, 65504)))
+    assert _native.device_status() == 0

@@ -182,3 +182,32 @@ def test_vllm_method_with_zero_points(plugin, single_rank_tp, cuda):
     y = method.apply(layer, x)
     w = oracle.dequantize_weight(src.qweight, src.scales, src.zeros, 8, 4)
     assert oracle.rel_err(y.cpu(), oracle.linear_fp32_accumulate(x.cpu(), w)) <= 1e-2
+
+
+@pytest.mark.gpu
+def test_vllm_method_with_zero_points_and_a_large_batch(plugin, single_rank_tp, cuda):
+    # wide enough for the tensor cores at this batch; calls that follow one another at once give what single ones give
+    from matgptq_b200 import _native, synth
+    cfg = plugin.MatGPTQConfig.from_config({"group_size": 128, "master_bitwidth": 8, "inference_bitwidth": 4,
+                                            "quant_dtype": "bfloat16", "modules_to_not_convert": ["lm_head", "norm"],
+                                            "zero_points": True})
+    method = plugin.MatGPTQLinearMethod(cfg, "model.layers.0.mlp.down_proj")
+    n_out, n_in, m = 4096, 4096, 72
+    layer = _FakeLinear()
+    method.create_weights(layer, n_in, [n_out], n_in, n_out, torch.bfloat16, weight_loader=lambda *a, **k: None)
+    src = synth.make_layer(n_out, n_in, 128, seed=8, sym=False, dtype=torch.bfloat16)
+    for name, value in (("qweight", src.qweight), ("scales", src.scales), ("zeros", src.zeros)):
+        getattr(layer, name).data.copy_(value)
+    layer.to(cuda)
+    method.process_weights_after_loading(layer)
+    x = synth.make_activations(m, n_in, seed=1, dtype=torch.bfloat16, device=cuda)
+    w = oracle.dequantize_weight(src.qweight, src.scales, src.zeros, 8, 4).to(cuda)
+    y = x
+    for _ in range(3):
+        ref = y.float() @ w.float().t()
+        z = method.apply(layer, y)
+        assert ((z.float() - ref).abs().max() / ref.abs().max()).item() <= 1e-2
+        y = z
+    chained = method.apply(layer, method.apply(layer, method.apply(layer, x)))
+    assert torch.equal(chained, y)
+    assert _native.device_status() == 0
