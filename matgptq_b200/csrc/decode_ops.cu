@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(256) silu_mul_vec_kernel(const T *__restrict__
 // mask [S, keys] in the model dtype for scores that are added up: 0 where a key is at or before the query's position, -inf
 // behind it.  Eight keys a thread with one 16-byte store where keys % 8 == 0.  Bound by latency (half a KB for a decode step):
 // one launch in the chain for the four elementwise ones that torch made of it (four 8B layers: a decode step at batch 1
-// 253.1 -> 247.0 us, at batch 32 466.8 -> 461.1).
+// 251 -> 247 us; at batch 32, 467 -> 463, within what runs differ by).
 template <typename T>
 __global__ void __launch_bounds__(128) causal_mask_kernel(const long long *__restrict__ positions, T *__restrict__ mask, int seq, int keys) {
   pdl_prologue();

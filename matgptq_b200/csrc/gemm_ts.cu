@@ -1,4 +1,4 @@
-// Tensor-core path with zero points, for every batch above 16 rows: tcgen05.mma with the WEIGHTS IN TENSOR MEMORY, scales and
+// Tensor-core path with zero points, above 16 rows where the GEMV's passes do not run side by side: tcgen05.mma with the WEIGHTS IN TENSOR MEMORY, scales and
 // zero points applied outside the product.
 //
 //   y[m, n] = 2^(8-b) * sum_g s[n, g] * (sum_{k in g} (code - Z) x[m, k]  -  z'[n, g] * sum_{k in g} x[m, k])
@@ -7,7 +7,7 @@
 // layout (16 out-features each) and a batch block; a pipeline stage is a block of 128 in-features:
 //
 //   * sixteen producer warps decode their tiles' blocks to the exact integers (code - Z), two instructions per pair of
-//     weights, and store them with tcgen05.st as the A operand in tensor memory, so that the weights do not pass through
+//     weights (five for 8-bit codes in bf16), and store them with tcgen05.st as the A operand in tensor memory, so that the weights do not pass through
 //     shared memory (written and read there they take 512 of its cycles for every 256 x 64 weights).  The packed layout gives a
 //     lane eight neighbouring in-features of a row, the store puts pairs of words side by side, and so it fixes an order of the
 //     in-features of its own;
@@ -25,10 +25,11 @@
 // until its copies and MMAs have ended (again with a limit), and tensor memory is freed on every path.
 //
 // The tiles of gemm_tc.cu hold scale * (code - zero) rounded to 16 bits, 1.4 times the error; the GEMV
-// scales in fp32 but takes a pass, with its own decoding, for every 16 rows.  What bounds it: a launch takes about 4 us around
-// its main loop (6 to 7 with a cluster's reduction); a block of 128 in-features takes 0.35 us for 8 tiles, the time in which the
-// issuing warp gets through two waits (90 cycles each, also when nothing has to be waited for), a request, eight MMAs and a
-// commit, or 0.6 us for 16 tiles, the issue slots of their decoding.
+// scales in fp32 but takes a pass, with its own decoding, for every 16 rows.  What bounds it (B200, from the launches that the plan
+// below is fitted to): a launch takes 4 to 6 us around its main loop, a cluster's reduction included; a block of 128 in-features
+// takes 0.8 us for 8 row tiles at 32 batch rows and 1.0 at 64 with groups of 128, 1.3 and 1.8 with groups of 32, 0.5 and 0.6 with
+// one scale per row.  The difference is the scaling and the sums of the activations, a chain of waits between the warps: at
+// 4096 x 4096, 128 rows, 4 bits, 22.2 us, the tensor pipe is busy 15 % of the time and 0.44 instructions are issued a cycle.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -206,8 +207,10 @@ __global__ void __launch_bounds__(kTsWarps * 32, 1) gemm_ts_kernel(const TsParam
   // kernel may take longer than the limit of such a wait.
   asm volatile("griddepcontrol.launch_dependents;");
 
-  // With K split the B stages hold [batch row][128 x row blocks out-feature slots] of sums once the last group is complete
-  // (and with it everything that reads a stage: the last sums of activations come before the barrier of their block).
+  // With K split the B stages, and where these are fewer than the sums need (16 row tiles) the first raw stages behind them,
+  // hold [batch row][128 x row blocks out-feature slots] of sums once the last group is complete (and with it everything that
+  // writes or reads a stage: every raw stage has been copied by then, and the last sums of activations come before the barrier
+  // of their block).
   float *staging = reinterpret_cast<float *>(base_ptr + kTsOffStages);
   const int slots = 128 * rbs;
   bool failed = false;
